@@ -1079,3 +1079,24 @@ def test_attention_kernels_at_random_shapes(K, err):
         assert e < 1.5e-2, (label, e)
         worst = max(worst, e)
     print(f"worst row error {worst:.2e}")
+
+
+# the FP32 kernel's rows per tile (1 to 16 by one warp's width, then 32 to 128), remainders of rows, columns and of the
+# inner dimension's blocks of 32, one slice of it and several, uneven ones among them
+@pytest.mark.parametrize("N,K_", [(120, 32), (257, 36), (130, 1096), (2048, 2048), (384, 6148), (5000, 260)])
+def test_gemm_f32_tiles(K, N, K_):
+    rows = (1, 2, 3, 5, 9, 16, 17, 33, 49, 65, 81, 97, 113, 128, 129, 300)
+    g = torch.Generator(device=DEV)
+    g.manual_seed(N)
+    a = torch.randn(max(rows), K_ + 4, generator=g, device=DEV)[:, :K_]          # (rows further apart than they are long)
+    w, bias = torch.randn(N, K_, generator=g, device=DEV), torch.randn(N, generator=g, device=DEV)
+    want = a.double() @ w.double().T + bias.double()
+    first = None
+    for m in rows:
+        out = torch.full((m + 1, N), 7.0, device=DEV)
+        K.gemm_simt(a[:m], w, bias, out[:m])
+        # the largest of the errors of sums of K products of unit variance, against the largest result
+        assert rel_err(out[:m], want[:m]) < acc_tol(K_)
+        assert bool((out[m] == 7.0).all())
+        first = out[:1].clone() if first is None else first
+        assert torch.equal(out[:1], first)               # whatever the batch
