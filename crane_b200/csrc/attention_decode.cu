@@ -62,6 +62,9 @@ struct FusedArgs {
     int cross;                      // (the plain form only) a CTA per (slice, pair of key/value heads, request):
                                     // queries and keys of the first, values of the second; always through the
                                     // scratch memory, and the merge kernel writes float [row][nq][nkv][d]
+    int* tickets;                   // entries of very different lengths (see balanced_slices): [entries][nkv] zeros, or null
+    int base_splits;                // the slices that entries of equal length would take
+    int slots;                      // CTAs that fit on the device at once
 };
 
 // A single element of the raw product (see raw2 for pairs).
@@ -576,13 +579,62 @@ __device__ __forceinline__ uint32_t sw_off(int row, int chunk) {
     return (uint32_t)((chunk >> 3) * HALF_TILE_BYTES + row * 128 + (((chunk & 7) ^ (row & 7)) << 4));
 }
 
+// An 8 x 8 matrix of 16-bit elements, lane holding row lane / 4, columns 2 (lane % 4) and the one after: its transpose.
+__device__ __forceinline__ uint32_t transposed_8x8(uint32_t v) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+
+// Slices of an entry of `n_tiles` tiles among entries of one token each (at most MAX_BALANCED): the longest one takes j
+// of at most n_splits slices, an entry of half its length half as many, with the largest j for which all slices
+// have a place on the device at once, at least `base`.  All lanes of a warp together.
+constexpr int MAX_BALANCED = 128;
+__device__ __forceinline__ int balanced_slices(int n_tiles, const int* __restrict__ cu_q, const int* __restrict__ kv_len,
+                                               int n_entries, int window, int nkv, int n_splits, int base, int slots, int lane) {
+    unsigned tiles[MAX_BALANCED / 32], longest = 1;
+#pragma unroll
+    for (int i = 0; i < MAX_BALANCED / 32; ++i) {
+        const int e = lane + 32 * i;
+        tiles[i] = 0;
+        if (e < n_entries && cu_q[e + 1] - cu_q[e] == 1) {
+            const int pos = kv_len[e] - 1, lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+            tiles[i] = (unsigned)(pos / TILE - lo / TILE + 1);
+        }
+        longest = max(longest, tiles[i]);
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    int j = n_splits;
+    for (; j > base; --j) {
+        unsigned all = 0;
+#pragma unroll
+        for (int i = 0; i < MAX_BALANCED / 32; ++i) all += (tiles[i] * j + longest - 1) / longest;
+        if (__reduce_add_sync(0xffffffffu, all) * nkv <= (unsigned)slots) break;
+    }
+    return max(1, (int)(((unsigned)n_tiles * j + longest - 1) / longest));
+}
+
 // CLUSTER: the CTAs of the slices of one (request, kv head) form a thread-block cluster (at most
 // 8 slices) and merge their results themselves through distributed shared memory: every CTA
 // leaves (max, sum, unnormalised output) of its slice in its own shared memory, and after a
 // cluster barrier each CTA works out its share of the output columns from all slices, in slice
 // order.  No scratch memory, no second kernel (a kernel of its own costs its place in the chain
 // of dependent launches, about 3 us per layer here, whatever little it does).
-template <bool FUSED, bool CLUSTER, bool GENERAL>
+//
+// BALANCED: entries of very different lengths.  With as many slices for every entry the longest one's are
+// what the kernel lasts (21 requests of 128 to 4,096 keys, 8 kv heads, 110 MB of keys and values: 168 CTAs, one
+// slice each, 86 us; 30 us balanced, 27 us with EIGHT as well).  Here an entry's slices are in proportion to its length, at most the grid's, the
+// others leave at once, and the CTA that finishes last merges an entry's slices from scratch memory (a
+// cluster would hold places for the slices that are not there).
+//
+// EIGHT: groups of at most 8 query heads.  The group then rides on the 8-wide side of the MMA and the keys (and, for the
+// output, the head's elements) on the 16-wide one: half the MMAs and half the exponentials of the form with the group
+// in 16 rows, most of which are empty.  The weights come out of the first product as (key, head) and enter
+// the second as (head, key): `movmatrix` turns them.  A CTA has two warps, each on a scheduler of its own, and the 64 dependent
+// MMAs of a tile were what it lasted, so that anything less than two CTAs on every SM fell short of the memory's rate.  One
+// launch, us, before / after: 24 requests of 4,096 keys, 8 kv heads (192 CTAs) 88 / 70; 48 of 4,096, 4 kv heads
+// 88 / 71; 8 of 8,192, 4 kv heads (8 slices) 27.0 / 26.2; 1 of 8,192 12.0 / 10.8.
+template <bool FUSED, bool CLUSTER, bool GENERAL, bool BALANCED, bool EIGHT>
 __global__ void __launch_bounds__(WARPS * 32)
 paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
                              const __grid_constant__ CUtensorMap v_map,
@@ -618,7 +670,10 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
 
     const int first_tile = lo / TILE;
     const int n_tiles = pos / TILE - first_tile + 1;
-    const int per_split = (n_tiles + n_splits - 1) / n_splits;
+    const int used = BALANCED ? balanced_slices(n_tiles, cu_q, kv_len, (int)gridDim.z, window, nkv, n_splits, fa.base_splits,
+                                                fa.slots, lane) : n_splits;
+    if (BALANCED && split >= used) return;         // (the whole CTA, before it waits for or touches anything)
+    const int per_split = (n_tiles + used - 1) / used;
     const int tile_begin = first_tile + split * per_split;
     const int tile_end = min(first_tile + n_tiles, tile_begin + per_split);
     const int n_my = max(0, (tile_end - tile_begin - warp + WARPS - 1) / WARPS);   // this warp's tiles
@@ -803,10 +858,13 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
         }
     }
 
-    float o[DN][4];
+    // (lane: rows lane / 4 and lane / 4 + 8, columns 2 (lane % 4) and the one after, of every 16 x 8 piece)
+    constexpr int OT = EIGHT ? DN / 2 : DN;                     // pieces of the output: elements x heads, or heads x elements
+    float o[OT][4];
 #pragma unroll
-    for (int i = 0; i < DN; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};     // m: unscaled maximum of the raw scores
+    for (int i = 0; i < OT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    // of the lane's two heads (columns, or rows without EIGHT); m: unscaled maximum of the raw scores
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 
     // per-lane parts of the ldmatrix addresses
     const int mi = lane >> 3, mr = lane & 7;
@@ -852,10 +910,13 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
             }
         }
 
-        // ---- scores: 16 rows x 32 keys ----
-        float s[4][4];
+        // ---- scores: 16 rows x 32 keys, or 32 keys x 8 rows ----
+        constexpr int ST = EIGHT ? 2 : 4;
+        float s[ST][4], odd[2][4];                              // (EIGHT: the odd pieces of 16 elements apart, for shorter chains)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+        for (int nt = 0; nt < ST; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) odd[nt][0] = odd[nt][1] = odd[nt][2] = odd[nt][3] = 0.f;
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
 #pragma unroll
@@ -865,30 +926,47 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
                                       ((uint32_t)(((ks & 3) * 2) << 4) ^ k_x);
                 uint32_t b0, b1, b2, b3;
                 ldmatrix_x4(addr, b0, b1, b2, b3);
-                mma_bf16(s[half * 2], qf[ks], b0, b1);
-                mma_bf16(s[half * 2 + 1], qf[ks], b2, b3);
+                if (EIGHT) {
+                    const uint32_t keys[4] = {b0, b2, b1, b3};
+                    if (ks & 1) mma_bf16(odd[half], keys, qf[ks][0], qf[ks][2]);
+                    else mma_bf16(s[half], keys, qf[ks][0], qf[ks][2]);
+                } else {
+                    mma_bf16(s[half * 2 % ST], qf[ks], b0, b1);
+                    mma_bf16(s[(half * 2 + 1) % ST], qf[ks], b2, b3);
+                }
             }
         }
-        // ---- running softmax ----
-        if (edge) {
-            const int key0 = ti * TILE + (lane & 3) * 2;
+        if (EIGHT) {
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s[nt][c] += odd[nt][c];
+        }
+        // ---- running softmax (element c of a piece belongs to the lane's head HEAD(c)) ----
+        auto head_of = [](int c) { return EIGHT ? c & 1 : c >> 1; };
+        if (edge) {
+            const int key0 = ti * TILE + (EIGHT ? lane >> 2 : (lane & 3) * 2);
+#pragma unroll
+            for (int nt = 0; nt < ST; ++nt)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const int j = key0 + nt * 8 + (c & 1);
+                    const int j = key0 + (EIGHT ? nt * 16 + (c >> 1) * 8 : nt * 8 + (c & 1));
                     if (j < lo || j > pos) s[nt][c] = -INFINITY;
                 }
         }
         float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < ST; ++nt)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) mx[c >> 1] = fmaxf(mx[c >> 1], s[nt][c]);
+            for (int c = 0; c < 4; ++c) mx[head_of(c)] = fmaxf(mx[head_of(c)], s[nt][c]);
         float m_new[2], base[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            m_new[h] = fmaxf(m[h], quad_max(mx[h]));
+            if (EIGHT) {
+#pragma unroll
+                for (int d = 4; d < 32; d <<= 1) mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], d));
+            }
+            m_new[h] = fmaxf(m[h], EIGHT ? mx[h] : quad_max(mx[h]));
             base[h] = (m_new[h] == -INFINITY) ? 0.f : m_new[h] * scale_log2;
         }
         if (__any_sync(0xffffffffu, m_new[0] != m[0] || m_new[1] != m[1])) {
@@ -900,19 +978,18 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
                 l[h] *= corr[h];
             }
 #pragma unroll
-            for (int i = 0; i < DN; ++i) {
-                o[i][0] *= corr[0]; o[i][1] *= corr[0];
-                o[i][2] *= corr[1]; o[i][3] *= corr[1];
-            }
+            for (int i = 0; i < OT; ++i)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) o[i][c] *= corr[head_of(c)];
         }
         float rs[2] = {0.f, 0.f};
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < ST; ++nt)
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const float p = exp2f(fmaf(s[nt][c], scale_log2, -base[c >> 1]));
+                const float p = exp2f(fmaf(s[nt][c], scale_log2, -base[head_of(c)]));
                 s[nt][c] = p;
-                rs[c >> 1] += p;
+                rs[head_of(c)] += p;
             }
         l[0] += rs[0];
         l[1] += rs[1];
@@ -920,10 +997,15 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
             uint32_t pf[4];
-            pf[0] = pack_bf16(s[2 * kk][0], s[2 * kk][1]);
-            pf[1] = pack_bf16(s[2 * kk][2], s[2 * kk][3]);
-            pf[2] = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]);
-            pf[3] = pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+            if (EIGHT) {
+                pf[0] = transposed_8x8(pack_bf16(s[kk][0], s[kk][1]));       // keys 0..7 of the 16, then 8..15
+                pf[1] = transposed_8x8(pack_bf16(s[kk][2], s[kk][3]));
+            } else {
+                pf[0] = pack_bf16(s[2 * kk % ST][0], s[2 * kk % ST][1]);
+                pf[1] = pack_bf16(s[2 * kk % ST][2], s[2 * kk % ST][3]);
+                pf[2] = pack_bf16(s[(2 * kk + 1) % ST][0], s[(2 * kk + 1) % ST][1]);
+                pf[3] = pack_bf16(s[(2 * kk + 1) % ST][2], s[(2 * kk + 1) % ST][3]);
+            }
 #pragma unroll
             for (int dn = 0; dn < DN; dn += 2) {
                 // matrices: (keys +0..7, d dn), (keys +8..15, d dn), (keys +0..7, d dn+1), (keys +8..15, d dn+1)
@@ -931,8 +1013,13 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
                                       ((uint32_t)((dn & 7) << 4) ^ v_x);
                 uint32_t b0, b1, b2, b3;
                 ldmatrix_x4_trans(addr, b0, b1, b2, b3);
-                mma_bf16(o[dn], pf, b0, b1);
-                mma_bf16(o[dn + 1], pf, b2, b3);
+                if (EIGHT) {
+                    const uint32_t elements[4] = {b0, b2, b1, b3};
+                    mma_bf16(o[dn / 2], elements, pf[0], pf[1]);
+                } else {
+                    mma_bf16(o[dn % OT], pf, b0, b1);
+                    mma_bf16(o[(dn + 1) % OT], pf, b2, b3);
+                }
             }
         }
         __syncwarp();
@@ -942,8 +1029,15 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
         if (lane == 0) atomicOr(err, CRANE_ERR_WAIT_TIMEOUT);
         for (int i = 0; i < 64; ++i) __nanosleep(1000);     // copies may still be landing
     }
-    l[0] = quad_sum(l[0]);
-    l[1] = quad_sum(l[1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (EIGHT) {
+#pragma unroll
+            for (int d = 4; d < 32; d <<= 1) l[h] += __shfl_xor_sync(0xffffffffu, l[h], d);
+        } else {
+            l[h] = quad_sum(l[h]);
+        }
+    }
     // from here on the maximum counts in the units of the scaled scores
     m[0] *= scale_log2;
     m[1] *= scale_log2;
@@ -957,13 +1051,26 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
     {
         const int r0 = lane >> 2, c0 = (lane & 3) * 2;
 #pragma unroll
-        for (int dn = 0; dn < DN; ++dn) {
-            float* p0 = sm_o + ((warp * 16 + r0) * D) + dn * 8 + c0;
-            float* p1 = sm_o + ((warp * 16 + r0 + 8) * D) + dn * 8 + c0;
-            p0[0] = o[dn][0]; p0[1] = o[dn][1];
-            p1[0] = o[dn][2]; p1[1] = o[dn][3];
+        for (int dn = 0; dn < OT; ++dn) {
+            if (EIGHT) {
+                float* p0 = sm_o + (warp * 16 + c0) * D + dn * 16 + r0;
+                p0[0] = o[dn][0]; p0[D] = o[dn][1];
+                p0[8] = o[dn][2]; p0[D + 8] = o[dn][3];
+            } else {
+                float* p0 = sm_o + ((warp * 16 + r0) * D) + dn * 8 + c0;
+                float* p1 = sm_o + ((warp * 16 + r0 + 8) * D) + dn * 8 + c0;
+                p0[0] = o[dn][0]; p0[1] = o[dn][1];
+                p1[0] = o[dn][2]; p1[1] = o[dn][3];
+            }
         }
-        if ((lane & 3) == 0) {
+        if (EIGHT) {
+            if (lane < 4)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    sm_ml[(warp * 16 + c0 + h) * 2] = m[h];
+                    sm_ml[(warp * 16 + c0 + h) * 2 + 1] = l[h];
+                }
+        } else if ((lane & 3) == 0) {
             sm_ml[(warp * 16 + r0) * 2] = m[0];      sm_ml[(warp * 16 + r0) * 2 + 1] = l[0];
             sm_ml[(warp * 16 + r0 + 8) * 2] = m[1];  sm_ml[(warp * 16 + r0 + 8) * 2 + 1] = l[1];
         }
@@ -983,7 +1090,7 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
             O += f * sm_o[(w * 16 + r) * D + c];
         }
         const int h = g * n_rep + r;
-        if (n_splits == 1 && !fa.cross) {
+        if (used == 1 && !fa.cross) {
             out[((long long)t * nq + h) * D + c] = __float2bfloat16_rn(finish_out(fa, t, h, D, c, O, L, mb));
         } else if (CLUSTER) {
             cl_o[r * D + c] = O;
@@ -1035,6 +1142,45 @@ paged_decode_attn_tma_kernel(const __grid_constant__ CUtensorMap k_map,
         // nobody leaves while a CTA of the cluster may still read its shared memory
         asm volatile("barrier.cluster.arrive.release.aligned;\n"
                      "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    if (BALANCED && used > 1) {
+        // the CTA that finds all others' results written adds the slices up, in slice order
+        __shared__ int ticket;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) ticket = atomicAdd(fa.tickets + e * nkv + g, 1);
+        __syncthreads();
+        if (ticket != used - 1) return;
+        if (threadIdx.x == 0) fa.tickets[e * nkv + g] = 0;               // for the next launch
+        __threadfence();
+        for (int idx = threadIdx.x; idx < n_rep * D / 4; idx += WARPS * 32) {
+            const int r = idx / (D / 4), c = idx % (D / 4) * 4, h = g * n_rep + r;
+            const long long base = ((long long)e * nq + h) * n_splits;
+            float2 ml[8];
+            float4 ov[8];
+#pragma unroll
+            for (int sp = 0; sp < 8; ++sp) {
+                ml[sp] = sp < used ? __ldcg((const float2*)(part_ml + (base + sp) * 2)) : make_float2(-INFINITY, 0.f);
+                ov[sp] = sp < used ? __ldcg((const float4*)(part_o + (base + sp) * D + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            float M = -INFINITY;
+#pragma unroll
+            for (int sp = 0; sp < 8; ++sp) M = fmaxf(M, ml[sp].x);
+            const float mb = (M == -INFINITY) ? 0.f : M;
+            float L = 0.f;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int sp = 0; sp < 8; ++sp) {
+                const float f = exp2f(ml[sp].x - mb);                    // 0 beyond the slices there are
+                L += f * ml[sp].y;
+                acc.x += f * ov[sp].x; acc.y += f * ov[sp].y; acc.z += f * ov[sp].z; acc.w += f * ov[sp].w;
+            }
+            __nv_bfloat16* to = out + ((long long)t * nq + h) * D + c;
+            *(__nv_bfloat162*)to = __floats2bfloat162_rn(finish_out(fa, t, h, D, c, acc.x, L, mb),
+                                                         finish_out(fa, t, h, D, c + 1, acc.y, L, mb));
+            *(__nv_bfloat162*)(to + 2) = __floats2bfloat162_rn(finish_out(fa, t, h, D, c + 2, acc.z, L, mb),
+                                                               finish_out(fa, t, h, D, c + 3, acc.w, L, mb));
+        }
     }
 }
 
@@ -1148,6 +1294,12 @@ EncodeTiledFn encode_fn() {
     }
     return fn;
 }
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
 // CRANE_DECODE_TMA=0 keeps the cp.async kernel at head size 128 too.
 bool tma_path_enabled() {
     static int on = -1;
@@ -1180,7 +1332,7 @@ bool pool_map(CUtensorMap* map, const void* pool, long long rows, int box_rows) 
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <bool FUSED, bool GENERAL>
+template <bool FUSED, bool GENERAL, bool EIGHT>
 int launch_decode_tma(const void* q, void* out, float* part_o, float* part_ml, const void* k_pool,
                       const void* v_pool, const int* cu_q, const int* kv_len, const int* block_table,
                       int max_blocks, int num_pages, int page_size, int nq, int nkv, int window,
@@ -1195,8 +1347,20 @@ int launch_decode_tma(const void* q, void* out, float* part_o, float* part_ml, c
     const int box_rows = page_size < TILE ? page_size : TILE;
     if (!pool_map(&km, k_pool, rows, box_rows) || !pool_map(&vm, v_pool, rows, box_rows))
         return (int)cudaErrorInvalidValue;
+    if (fa.tickets != nullptr) {
+        auto kern = paged_decode_attn_tma_kernel<FUSED, false, GENERAL, true, EIGHT>;
+        static bool configured = false;
+        if (!configured) {
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+                return (int)cudaGetLastError();
+            configured = true;
+        }
+        return crane_launch(kern, grid, dim3(WARPS * 32), smem, st, km, vm, (const __nv_bfloat16*)q,
+                            (__nv_bfloat16*)out, part_o, part_ml, cu_q, kv_len, block_table, max_blocks,
+                            num_pages, page_size, nq, nkv, window, scale * 1.4426950408889634f, n_splits, err, fa);
+    }
     if (cluster) {
-        auto kern = paged_decode_attn_tma_kernel<FUSED, true, GENERAL>;
+        auto kern = paged_decode_attn_tma_kernel<FUSED, true, GENERAL, false, EIGHT>;
         static bool configured = false;
         if (!configured) {
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
@@ -1208,7 +1372,7 @@ int launch_decode_tma(const void* q, void* out, float* part_o, float* part_ml, c
                                     block_table, max_blocks, num_pages, page_size, nq, nkv, window,
                                     scale * 1.4426950408889634f, n_splits, err, fa);
     }
-    auto kern = paged_decode_attn_tma_kernel<FUSED, false, GENERAL>;
+    auto kern = paged_decode_attn_tma_kernel<FUSED, false, GENERAL, false, EIGHT>;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
@@ -1225,7 +1389,7 @@ template <int D, bool FUSED, bool GENERAL>
 int launch_decode(const void* q, void* out, float* part_o, float* part_ml, const void* k_pool,
                   const void* v_pool, const int* cu_q, const int* kv_len, const int* block_table,
                   int max_blocks, int num_pages, int page_size, int n_entries, int nq, int nkv,
-                  int window, float scale, int n_splits, int* err, const FusedArgs& fa, cudaStream_t st) {
+                  int window, float scale, int n_splits, int* err, const FusedArgs& args, cudaStream_t st) {
     constexpr int tiles = WARPS * NSTAGE * 2 * TILE * Tile<D>::ROW_BYTES + (FUSED ? 16 * D * 2 : 0);
     constexpr int merge = WARPS * 16 * (D + 2) * 4;
     constexpr int smem = tiles > merge ? tiles : merge;
@@ -1236,20 +1400,31 @@ int launch_decode(const void* q, void* out, float* part_o, float* part_ml, const
             return (int)cudaGetLastError();
         configured = true;
     }
-    const int cross = (!FUSED && fa.cross) ? 1 : 0;
+    const int cross = (!FUSED && args.cross) ? 1 : 0;
     const int nq_out = cross ? nq * nkv : nq;       // heads of the merged output
-    dim3 grid(n_splits, cross ? nkv * nkv : nkv, n_entries);
     // pages of whole tiles, or tiles of whole pages (8 or 16 tokens: a piece of a tile is then a multiple
     // of the 1024 bytes the swizzle pattern repeats after)
     const bool pages_fit = page_size % TILE == 0 || (page_size >= 8 && TILE % page_size == 0);
-    if (D == D128 && pages_fit && tma_path_enabled()) {
+    const bool by_tma = D == D128 && pages_fit && tma_path_enabled();
+    FusedArgs fa = args;
+    if (fa.tickets != nullptr && (!by_tma || cross || n_splits < 2 || n_splits > 8 || n_entries > MAX_BALANCED)) {
+        fa.tickets = nullptr;                        // as many slices for every entry
+        n_splits = fa.base_splits;
+    }
+    dim3 grid(n_splits, cross ? nkv * nkv : nkv, n_entries);
+    if (by_tma) {
         // 2 to 8 slices merge themselves in a cluster; more go through scratch memory and a second kernel
-        const bool cluster = n_splits > 1 && n_splits <= 8 && !cross && cluster_merge_enabled();
-        const int rc = launch_decode_tma<FUSED, GENERAL>(q, out, part_o, part_ml, k_pool, v_pool, cu_q, kv_len,
-                                                block_table, max_blocks, num_pages, page_size, nq, nkv,
-                                                window, scale, n_splits, err, fa, grid, cluster, st);
+        const bool cluster = n_splits > 1 && n_splits <= 8 && !cross && fa.tickets == nullptr && cluster_merge_enabled();
+        // Groups of more than 8 heads need the 16-row form; so, by measurement, does one slice each for (request, kv head)s
+        // that take more than four fifths of the places: the memory is then the bound from beginning to end, and CTAs
+        // that can run ahead only end less evenly (64 requests of 8,192 keys, 4 kv heads: 7.10 ms a step, 7.25 with the
+        // 8-column form; 56 requests of 4,096 keys, one launch: 88 us, 73).
+        const bool crowded = n_splits == 1 && 5 * n_entries * nkv > 4 * 2 * sm_count();
+        auto launch = nq / nkv <= 8 && !crowded ? launch_decode_tma<FUSED, GENERAL, true> : launch_decode_tma<FUSED, GENERAL, false>;
+        const int rc = launch(q, out, part_o, part_ml, k_pool, v_pool, cu_q, kv_len, block_table, max_blocks, num_pages,
+                              page_size, nq, nkv, window, scale, n_splits, err, fa, grid, cluster, st);
         if (rc != 0) return rc;
-        if ((n_splits > 1 && !cluster) || cross)
+        if ((n_splits > 1 && !cluster && fa.tickets == nullptr) || cross)
             return crane_launch(decode_merge_kernel, dim3(n_entries, nq_out), dim3(D >= 128 ? 128 : 64), 0, st,
                                 (const float*)part_o, (const float*)part_ml, (__nv_bfloat16*)out, cu_q, nq_out,
                                 D, n_splits, fa, cross);
@@ -1329,6 +1504,9 @@ CRANE_API int crane_paged_decode_attention_supports(int d, int nq, int nkv) {
 // when n_splits > 1.  cross != 0: `out` is float [rows][nq][nkv][d], every query head's weights
 // applied to the values of every key/value head; the scratch memory is always used and takes nkv
 // times as much.  sinks and the gate as in crane_paged_prefill_attention (neither with cross).
+// tickets (int [n_entries][nkv], zeros, left as zeros) != null: entries of very different lengths, which take up to
+// n_splits slices in proportion to their lengths (see balanced_slices; `slots` CTAs fit on the device at once); where the
+// kernel that does so does not apply, every entry takes base_splits.
 CRANE_API int crane_paged_decode_attention(const void* q, void* out, float* part_o, float* part_ml,
                                            const void* k_pool, const void* v_pool, const int* cu_q,
                                            const int* kv_len, const int* block_table, int max_blocks,
@@ -1336,9 +1514,10 @@ CRANE_API int crane_paged_decode_attention(const void* q, void* out, float* part
                                            int d, int window, float scale, int n_splits, int sink,
                                            const float* sinks, const void* gate, const float* gate_parts,
                                            int gate_n_parts, long long gate_stride, int gate_ld, int gate_off,
-                                           int cross, int* err, cudaStream_t st) {
+                                           int cross, int* tickets, int base_splits, int slots, int* err, cudaStream_t st) {
     if (n_entries <= 0) return 0;
     if (!crane_paged_decode_attention_supports(d, nq, nkv) || n_splits < 1 || n_splits > 64 ||
+        (tickets != nullptr && (base_splits < 1 || base_splits > n_splits || part_o == nullptr || part_ml == nullptr)) ||
         (cross && (part_o == nullptr || part_ml == nullptr || gate_ld > 0 || sinks != nullptr)))
         return (int)cudaErrorInvalidValue;
     FusedArgs none = {};
@@ -1348,6 +1527,7 @@ CRANE_API int crane_paged_decode_attention(const void* q, void* out, float* part
     none.part_stride = gate_stride; none.qkv_stride = gate_ld;
     none.gate_off = gate_ld > 0 ? gate_off : -1;
     none.cross = cross ? 1 : 0;
+    none.tickets = tickets; none.base_splits = base_splits; none.slots = slots;
     return launch_for_head_size(d, 0, q, out, part_o, part_ml, k_pool, v_pool, cu_q, kv_len, block_table,
                                 max_blocks, num_pages, page_size, n_entries, nq, nkv, window, scale,
                                 n_splits, err, &none, st);
@@ -1366,10 +1546,11 @@ CRANE_API int crane_paged_decode_attention_fused(
     void* k_pool, void* v_pool, const int* cu_q, const int* kv_len,
     const int* block_table, int max_blocks, int num_pages, int page_size, int n_entries, int nq, int nkv,
     int d, int window, float scale, int n_splits, int rotary_dim, int interleaved, int norm_first,
-    float norm_offset, const float* sinks, int gate_off, int* err, cudaStream_t st) {
+    float norm_offset, const float* sinks, int gate_off, int* tickets, int base_splits, int slots, int* err, cudaStream_t st) {
     if (n_entries <= 0) return 0;
     if (rotary_dim <= 0) rotary_dim = d;
-    if (!crane_paged_decode_attention_supports(d, nq, nkv) || n_splits < 1 || n_splits > 64 || (d & 3) ||
+    if ((tickets != nullptr && (base_splits < 1 || base_splits > n_splits || part_o == nullptr || part_ml == nullptr)) ||
+        !crane_paged_decode_attention_supports(d, nq, nkv) || n_splits < 1 || n_splits > 64 || (d & 3) ||
         (qkv_stride & 1) || (part_stride & 1) || rotary_dim > d || (rotary_dim & 1))
         return (int)cudaErrorInvalidValue;
     FusedArgs fa = {};
@@ -1380,6 +1561,7 @@ CRANE_API int crane_paged_decode_attention_fused(
     fa.cos_tab = cos_tab; fa.sin_tab = sin_tab; fa.table_len = table_len; fa.q_norm_w = q_norm_w;
     fa.k_norm_w = k_norm_w; fa.eps = eps; fa.k_pool_w = (__nv_bfloat16*)k_pool;
     fa.v_pool_w = (__nv_bfloat16*)v_pool; fa.sinks = sinks; fa.gate_off = gate_off;
+    fa.tickets = tickets; fa.base_splits = base_splits; fa.slots = slots;
     return launch_for_head_size(d, 1, nullptr, out, part_o, part_ml, k_pool, v_pool, cu_q, kv_len,
                                 block_table, max_blocks, num_pages, page_size, n_entries, nq, nkv, window,
                                 scale, n_splits, err, &fa, st);
@@ -1452,6 +1634,7 @@ CRANE_API int crane_paged_decode_attention_noalloc(const void* q, void* out, con
     }
     return crane_paged_decode_attention(q, out, part_o, part_ml, k_pool, v_pool, cu_q, kv_len,
                                         block_table, max_blocks, num_pages, page_size, n_entries, nq,
-                                        nkv, d, window, scale, n_splits, 0, nullptr, nullptr, nullptr, 0, 0, 0, -1, 0, err, stream);
+                                        nkv, d, window, scale, n_splits, 0, nullptr, nullptr, nullptr, 0, 0, 0, -1, 0, nullptr, 0, 0, err,
+                                        stream);
 }
 #endif  // CRANE_HEAD_SIZE

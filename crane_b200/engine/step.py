@@ -35,6 +35,10 @@ from ..weights.safetensors_io import DictSource
 # ``Kernels.decode_splits``).
 SHORT_CONTEXT = 2048
 SHORT_GRAPH_KEY = 1 << 20
+# A decode step whose longest context is at least half as long again as the average (and long enough to matter):
+# its attention gives long contexts more key slices, in a kernel of its own, so its graphs are others.
+UNEVEN_GRAPH_KEY = 1 << 21
+UNEVEN_KEYS = 512
 # A step whose every entry has at most this many keys in all (whole short prompts).
 SHORT_PROMPT = 64
 
@@ -85,6 +89,7 @@ class StepContext:
                                 # an attention mixer may give them to its split-KV decode kernel and
                                 # the rest to its prefill kernel
     short_prompts: bool = False     # no entry has more than 64 keys in all (whole short prompts)
+    uneven: bool = False        # the entries of one token differ in length so much that their attention is balanced
     all_single: bool = False        # every entry has exactly one token (part of a padded step's shape)
 
 
@@ -316,6 +321,12 @@ class ModelRunner:
             one = cnt == 1
             if one.any() and int(m.view("kv_len", n_entries, False)[one].sum()) >= self.cfg.mixed_decode_min_keys:
                 singles = int(one.sum())
+        uneven = False
+        if not self.rt.exact:
+            held = m.view("kv_len", n_entries, False)[cnt == 1]
+            if held.size > 1 and (pad_to or singles):
+                longest = int(held.max())
+                uneven = longest >= UNEVEN_KEYS and 2 * longest * held.size > 3 * int(held.sum())
         # a small step with prompt portions: its rows are padded to a multiple of 64, its entries
         # and wanted places to a power of two, and from the second step of the same (rows,
         # entries, wanted, single-token entries) on a captured graph is replayed
@@ -331,7 +342,8 @@ class ModelRunner:
                      self._power_of_two(wanted, rows) if wanted else 0,
                      self._power_of_two(singles, self.cap_entries) if singles else 0,
                      1 if short_prompts else 0,
-                     1 if int(cnt.max()) == 1 else 0)     # nothing but single tokens: a decode step
+                     1 if int(cnt.max()) == 1 else 0,     # nothing but single tokens: a decode step
+                     1 if uneven else 0)
             seen = self._shape_seen.get(shape, 0) + 1
             self._shape_seen[shape] = seen
             if seen >= 2:
@@ -383,6 +395,7 @@ class ModelRunner:
         ctx.graph_key = key
         ctx.single_entries = singles
         ctx.short_prompts = short_prompts
+        ctx.uneven = uneven
         ctx.all_single = int(cnt.max()) == 1
         # While the device still runs the step before, the host launches this step's kernels
         # behind it at no cost, and launched one by one they ran a little faster than replayed
@@ -424,7 +437,8 @@ class ModelRunner:
                 # (a graph holds the number of key slices its attention was recorded with: short
                 # contexts, which take fewer, have graphs of their own)
                 short = ctx.max_kv_len <= SHORT_CONTEXT
-                return self._replay(ctx, ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0))[:ctx.real_entries]
+                return self._replay(ctx, ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
+                                    + (UNEVEN_GRAPH_KEY if ctx.uneven else 0))[:ctx.real_entries]
             if ctx.graph_key is not None and ctx.replay:
                 return self._replay(ctx, ctx.graph_key)[:ctx.real_want]
             return self.model.forward(ctx, self.pools.layers)[:ctx.real_want]

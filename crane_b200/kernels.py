@@ -31,11 +31,11 @@ _SIGNATURES = {
     "crane_gemm_bf16_pair": [P, P, P, P, I, I, I, L, L, L, I, I, I, I, I, P, P],
     "crane_paged_attention_simt": [I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P, P, P],
     "crane_paged_decode_attention_supports": [I, I, I],
-    "crane_paged_decode_attention": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, P, P, P, I, L, I, I, I, P, P],
+    "crane_paged_decode_attention": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, P, P, P, I, L, I, I, I, P, I, I, P, P],
     "crane_paged_prefill_attention_supports": [I, I, I],
     "crane_paged_prefill_attention": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, P, P, P, I, L, I, I, P, P, P],
     "crane_paged_decode_attention_fused": [P, P, I, L, I, I, I, P, P, I, P, P, F, P, P, P, P, P, P, P, P,
-                                           I, I, I, I, I, I, I, I, F, I, I, I, I, F, P, I, P, P],
+                                           I, I, I, I, I, I, I, I, F, I, I, I, I, F, P, I, P, I, I, P, P],
     "crane_prefill_attention_tc_supports": [I, I, I, I],
     "crane_prefill_attention_tc": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P, P, I, L, I, I, P, P],
     "crane_embed_bigram": [I, P, P, P, P, I, I, I, I, L, L, P, P, P, P, P, I, P, I, P, P],
@@ -1100,6 +1100,27 @@ class Kernels:
         return bool(self.lib.crane_paged_decode_attention_supports(d, nq, nkv))
 
     @staticmethod
+    def _balance(balance, n_entries: int, nkv: int):
+        if balance is None:
+            return [None, 0, 0]
+        tickets, base, slots = balance
+        assert tickets.dtype == torch.int32 and tickets.numel() >= n_entries * nkv and tickets.is_contiguous()
+        return [tickets.data_ptr(), int(base), int(slots)]
+
+    MOST_BALANCED = 128          # entries of a step whose slices the decode attention balances
+
+    @staticmethod
+    def balanced_most(base: int) -> int:
+        """The most key slices a (request, kv head) may take where the entries' lengths differ, ``base`` being what
+        entries of equal length take; 0: every entry takes ``base``.  Measured, one launch, contexts spread from a
+        thirty-second of the longest up to it (us, every entry ``base`` slices / at most 4 / 6 / 8 in proportion):
+        21 requests of up to 4,096 keys, 8 kv heads, base 1: 66 / 27 / 28 / 30; 40 of 3,000, 4 kv heads, base 1: 49 / 22 /
+        22 / 24; 48 of 4,096, 8 kv heads, base 2: 54 / 49 / 52 / 57; 14 of 6,000, 4 kv heads, base 4: 30 / 32 / 24 / 21; 8 of
+        8,192, 4 kv heads, base 8: 22 / - / - / 25 (as many slices as a cluster holds, and the merge in the cluster is the
+        cheaper one)."""
+        return max(4, 2 * base) if base <= 4 else 0
+
+    @staticmethod
     def _gate(gate):
         if gate is None:
             return [None, None, 0, 0, 0, 0]
@@ -1107,7 +1128,7 @@ class Kernels:
 
     def paged_decode_attention(self, q, out, k_pool, v_pool, cu_q, kv_len, block_table, page_size,
                                nq, nkv, d, window, scale, n_splits, part_o, part_ml, err, sink: bool = False,
-                               cross: bool = False, sinks=None, gate=None) -> None:
+                               cross: bool = False, sinks=None, gate=None, balance=None) -> None:
         """The entries of exactly one token (bfloat16); entries with more or no
         rows are skipped.  ``part_o`` [entries * nq * n_splits * d] and ``part_ml``
         [entries * nq * n_splits * 2] floats are scratch for n_splits > 1.  ``sink``: the
@@ -1116,7 +1137,8 @@ class Kernels:
         (for heads that exchange their weights); the scratch is always used and nkv times as large.
         ``sinks`` float [nq]: a candidate of that score without a value joins every softmax of its head.
         ``gate`` (product, its row length, column): the result is multiplied by the sigmoid of the product's columns
-        column + h d .. of the token's row."""
+        column + h d .. of the token's row.  ``balance`` (int32 zeros [entries, nkv], slices of entries of equal length,
+        CTAs that fit on the device): up to ``n_splits`` slices in proportion to the entries' lengths."""
         assert not cross or (out.dtype == torch.float32 and part_o is not None)
         n_entries = kv_len.shape[0]
         self.require_head_size(d)
@@ -1125,7 +1147,7 @@ class Kernels:
             v_pool.data_ptr(), cu_q.data_ptr(), kv_len.data_ptr(), block_table.data_ptr(),
             block_table.shape[1], k_pool.shape[0], page_size, n_entries, nq, nkv, d, int(window),
             float(scale), int(n_splits), 1 if sink else 0, _ptr(sinks), *self._gate(gate), 1 if cross else 0,
-            err.data_ptr(), self._stream(q)),
+            *self._balance(balance, n_entries, nkv), err.data_ptr(), self._stream(q)),
             "paged_decode_attention")
 
     def prefill_attention_supports(self, d: int, nq: int, nkv: int) -> bool:
@@ -1168,11 +1190,12 @@ class Kernels:
     def paged_decode_attention_fused(self, qkv: Act, qkv_cols, has_kv, cos, sin, q_norm_w, k_norm_w,
                                      eps, out, k_pool, v_pool, cu_q, kv_len, block_table, page_size,
                                      nq, nkv, d, window, scale, n_splits, part_o, part_ml, err,
-                                     rope=None, sinks=None, gate_off: int = -1) -> None:
+                                     rope=None, sinks=None, gate_off: int = -1, balance=None) -> None:
         """One token per entry, straight from the q/k/v product: rotary encoding,
         per-head norm, cache write and attention in one kernel, then the merge of
         the key slices.  ``rope`` as in ``rope_norm_cache``; ``sinks`` as in ``paged_decode_attention``;
-        ``gate_off`` >= 0: the result is multiplied by the sigmoid of the product's columns gate_off + h d .. ."""
+        ``gate_off`` >= 0: the result is multiplied by the sigmoid of the product's columns gate_off + h d .. .
+        ``balance`` as in ``paged_decode_attention``."""
         rd, inter, first, off = rope or (d, False, False, 0.0)
         whole, parts, n_parts, stride = _split(qkv)
         n_entries = kv_len.shape[0]
@@ -1184,8 +1207,8 @@ class Kernels:
             k_pool.data_ptr(), v_pool.data_ptr(), cu_q.data_ptr(), kv_len.data_ptr(),
             block_table.data_ptr(), block_table.shape[1], k_pool.shape[0], page_size, n_entries, nq,
             nkv, d, int(window), float(scale), int(n_splits), int(rd), 1 if inter else 0,
-            1 if first else 0, float(off), _ptr(sinks), int(gate_off), err.data_ptr(), self._stream(out)),
-            "paged_decode_attention_fused")
+            1 if first else 0, float(off), _ptr(sinks), int(gate_off), *self._balance(balance, n_entries, nkv),
+            err.data_ptr(), self._stream(out)), "paged_decode_attention_fused")
 
     # ---- sampling -------------------------------------------------------
     def repetition_penalty(self, logits, context, ctx_len, penalty) -> None:

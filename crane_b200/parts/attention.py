@@ -145,6 +145,17 @@ class GqaAttention(Part):
             return CacheNeed("none")
         return CacheNeed("kv", kv_heads=self.nkv, head_dim=self.d, window=self.window)
 
+    def _balance(self, ctx, rt, splits: int):
+        """(the decode attention's ``balance``, the most slices of an entry) for a step whose entries of one token
+        differ in length; (None, ``splits``) where every entry takes ``splits``."""
+        k = rt.kernels
+        most = k.balanced_most(splits) if getattr(ctx, "uneven", False) and ctx.n_entries <= k.MOST_BALANCED else 0
+        if not most or self.max_splits < most:
+            return None, splits
+        # (kept by the workspace: zeros, which every launch leaves as zeros)
+        tickets = rt.ws.zeros("attn_tickets", k.MOST_BALANCED, self.nkv, torch.int32)
+        return (tickets, splits, 2 * rt.num_sms), most
+
     def forward(self, h, ctx, cache, rt, hold: bool = False):
         n = h.shape[0]
         k = rt.kernels
@@ -169,14 +180,17 @@ class GqaAttention(Part):
             splits = k.decode_splits(ctx.n_entries, self.nkv, rt.num_sms, self.max_splits, max_keys=keys)
             # slices x entries never exceed two CTAs per SM, or the slices are 4 at most: that bounds
             # the slices' scratch rows
-            rows = self.nq * max(2 * rt.num_sms // self.nkv + 1, 4 * rt.max_decode_rows)
+            # (8 slices each where their number follows the entries' lengths)
+            rows = self.nq * max(2 * rt.num_sms // self.nkv + 1, 8 * rt.max_decode_rows)
+            balance, most = self._balance(ctx, rt, splits)
             part_o = rt.ws.get("attn_part_o", rows, self.d, torch.float32, cap=rows)
             part_ml = rt.ws.get("attn_part_ml", rows, 2, torch.float32, cap=rows)
             k.paged_decode_attention_fused(qkv, self.qkv_cols, self.own_kv, cos, sin, self.q_norm,
                                            self.k_norm, self.eps, o, cache.k, cache.v, ctx.cu_q,
                                            ctx.kv_len, table, cache.page_size, self.nq, self.nkv,
-                                           self.d, self.window, self.scale, splits, part_o, part_ml,
-                                           rt.err, rope=self.rope, sinks=self.sinks, gate_off=self.gate_off)
+                                           self.d, self.window, self.scale, most, part_o, part_ml,
+                                           rt.err, rope=self.rope, sinks=self.sinks, gate_off=self.gate_off,
+                                           balance=balance)
             rt.launches += 1 if splits <= 8 else 2     # the merge is a launch of its own above 8 slices
             return rt.linear(o, self.o_w, self.o_b, "attn_out", hold=hold)
         q = rt.ws.get("attn_q", n, self.nq * self.d, rt.dtype)
@@ -204,14 +218,15 @@ class GqaAttention(Part):
             else:
                 # at most 8 slices: at head size 128 they merge inside a cluster without scratch
                 splits = min(8, k.decode_splits(singles, self.nkv, rt.num_sms, self.max_splits))
+            balance, most = (None, splits) if decode else self._balance(ctx, rt, splits)
             part_o = part_ml = None
-            if splits > 1:
+            if most > 1:
                 rows = rt.max_decode_rows * self.nq * 32
                 part_o = rt.ws.get("attn_part_o", rows, self.d, torch.float32, cap=rows)
                 part_ml = rt.ws.get("attn_part_ml", rows, 2, torch.float32, cap=rows)
             k.paged_decode_attention(q, o, cache.k, cache.v, ctx.cu_q, ctx.kv_len, table,
                                      cache.page_size, self.nq, self.nkv, self.d, self.window,
-                                     self.scale, splits, part_o, part_ml, rt.err, sinks=self.sinks, gate=gate)
+                                     self.scale, most, part_o, part_ml, rt.err, sinks=self.sinks, gate=gate, balance=balance)
             rt.launches += 3 if splits > 1 else 2
             if decode:
                 return rt.linear(o, self.o_w, self.o_b, "attn_out", hold=hold)

@@ -1100,3 +1100,49 @@ def test_gemm_f32_tiles(K, N, K_):
         assert bool((out[m] == 7.0).all())
         first = out[:1].clone() if first is None else first
         assert torch.equal(out[:1], first)               # whatever the batch
+
+
+# lengths that differ: one long request among short ones, entries without a row, slices that fill the grid and entries of one
+# slice, groups of one and of several heads, a window, pages smaller than a tile, more entries than lanes
+@pytest.mark.parametrize("nq,nkv,page_size,window,base,most,lens", [
+    (16, 4, 64, 0, 1, 8, [4096, 70, 33, 1, 900, 257, 64, 31]), (32, 8, 64, 0, 1, 5, [2500, 0, 1200, 40, 0, 513, 700, 32, 5]),
+    (4, 4, 16, 200, 2, 8, [1500, 210, 3, 90]), (8, 2, 8, 0, 3, 3, [640, 33]),
+    (16, 4, 32, 0, 1, 4, [3000] + [17 + 13 * i for i in range(69)])])
+def test_decode_attention_balanced(K, err, nq, nkv, page_size, window, base, most, lens):
+    """Slices in proportion to the entries' lengths against the plain attention, plain and fused, launch after launch."""
+    d, slots = 128, 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    torch.manual_seed(len(lens))
+    live = [i for i, n in enumerate(lens) if n]
+    ks = [torch.randn(max(n, 1), nkv, d).bfloat16().float() for n in lens]
+    vs = [torch.randn(max(n, 1), nkv, d).bfloat16().float() for n in lens]
+    k_pool, v_pool, table = paged_cache(ks, vs, page_size, torch.bfloat16)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + (1 if n else 0))
+    q = torch.randn(len(live), nq, d, device=DEV).bfloat16()
+    want = torch.stack([attention_reference(q[cu[i]].float().cpu(), ks[i], vs[i], lens[i] - 1, window) for i in live])
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)                                 # noqa: E731
+    part_o = torch.full((len(lens) * nq * most, d), float("nan"), device=DEV)
+    part_ml = torch.full((len(lens) * nq * most, 2), float("nan"), device=DEV)
+    tickets = torch.zeros(len(lens), nkv, dtype=torch.int32, device=DEV)
+    for _ in range(2):
+        out = torch.full_like(q, float("nan"))
+        K.paged_decode_attention(q, out, k_pool, v_pool, i32(cu), i32(lens), table, page_size, nq, nkv, d, window, d ** -0.5,
+                                 most, part_o, part_ml, err, balance=(tickets, base, slots))
+        assert int(err.item()) == 0 and not bool(tickets.any())
+        assert rel_err(out.cpu(), want) < TOL[torch.bfloat16]
+    # the fused form: the newest position's key and value come from the product and go into their page
+    qkv = torch.cat([q.reshape(len(live), -1)] + [torch.stack([t[i][lens[i] - 1].reshape(-1) for i in live]).bfloat16().to(DEV)
+                                                  for t in (ks, vs)], dim=1).contiguous()
+    k2, v2 = k_pool.clone(), v_pool.clone()
+    for i in live:                                           # (what lies in the page before must not matter)
+        page, row = int(table[i, (lens[i] - 1) // page_size]), (lens[i] - 1) % page_size
+        k2[page, :, row] = 77.0
+        v2[page, :, row] = 77.0
+    out = torch.full_like(q, float("nan"))
+    K.paged_decode_attention_fused(qkv, qkv.shape[1], True, None, None, None, None, 0.0, out, k2, v2, i32(cu), i32(lens), table,
+                                   page_size, nq, nkv, d, window, d ** -0.5, most, part_o, part_ml, err,
+                                   balance=(tickets, base, slots))
+    assert int(err.item()) == 0 and not bool(tickets.any())
+    assert rel_err(out.cpu(), want) < TOL[torch.bfloat16]
+    assert torch.equal(k2, k_pool) and torch.equal(v2, v_pool)
