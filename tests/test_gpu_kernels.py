@@ -1146,3 +1146,32 @@ def test_decode_attention_balanced(K, err, nq, nkv, page_size, window, base, mos
     assert int(err.item()) == 0 and not bool(tickets.any())
     assert rel_err(out.cpu(), want) < TOL[torch.bfloat16]
     assert torch.equal(k2, k_pool) and torch.equal(v2, v_pool)
+
+
+# more rows than a step of few tokens: one and two pieces of four columns a thread, rows that do not fill the threads, a product
+# that comes whole, in one to five partial sums, or not at all
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n,hidden,parts", [(65, 96, 3), (70, 132, 0), (130, 2048, 4), (130, 2048, 0), (300, 2052, 1), (66, 3072, 5),
+                                            (257, 4096, 0), (65, 8192, 2), (65, 3072, -1)])
+def test_add_rmsnorm_many_rows(K, dtype, n, hidden, parts):
+    from crane_b200.kernels import Partials
+    g = torch.Generator(device=DEV)
+    g.manual_seed(hidden + n)
+    x, w = torch.randn(n, hidden, generator=g, device=DEV), 1 + 0.1 * torch.randn(hidden, generator=g, device=DEV)
+    delta, added = None, torch.zeros(n, hidden, device=DEV)
+    if parts == 0:
+        delta = torch.randn(n, hidden, generator=g, device=DEV).to(dtype)
+        added = delta.float()
+    elif parts > 0:
+        p = torch.randn(parts, n, hidden, generator=g, device=DEV)
+        delta, total = Partials(p), p[0].clone()
+        for i in range(1, parts):
+            total = total + p[i]
+        added = total.to(dtype).float()                      # rounded once, in slice order
+    want_x = x + added
+    got, out = x.clone(), torch.empty(n, hidden, device=DEV, dtype=dtype)
+    K.add_rmsnorm(got, delta, w, 1e-5, out)
+    assert torch.equal(got, want_x)
+    d = want_x.double()
+    want = d * torch.rsqrt((d * d).mean(-1, keepdim=True) + 1e-5) * w.double()
+    assert rel_err(out, want) < TOL[dtype]
