@@ -216,6 +216,17 @@ class Runtime:
                 tiles = (N + 127) // 128
                 # at most 8: the consumers of partial sums fetch eight slices at a time
                 slices = min(k.slices_for(tiles, K, self.num_sms), 8)
+                most = 2 * self.num_sms // (tiles * -(-M // 64))
+                if bn == 256 and most >= 1 and (most >= 3 or K // most <= 4096):
+                    # More than 128 tokens: tiles of 64, two CTAs an SM, fewer slices of the inner dimension, instead of
+                    # one tile of 256 (padded) tokens that takes an SM for itself and leaves up to 8 partial sums of
+                    # everything.  Where all tiles are there at once (else the weights came from DRAM once per tile of
+                    # tokens) and a CTA's share of the inner dimension is not long.  Whole prompts, ms: 1.8B sizes, 137
+                    # tokens 2.41 -> 2.08, 250 tokens 2.68 -> 2.21; 7B sizes, 250 tokens, down with 2 slices of 7,168
+                    # 5.01 -> 5.16, hence the second condition.
+                    bn = 64
+                    tiles *= -(-M // 64)
+                    slices = min(8, most, max(1, K // 256))
                 nxt = self._next_weights(w) if w.is_contiguous() else None
                 # Measured in whole decode steps (Hunyuan-1.8B sizes): a single token gains 2.4 % at a
                 # context of 2,048 and 4.6 % at 8,192; from two tokens on the hints cost 1 to 4 % (the
@@ -248,7 +259,23 @@ class Runtime:
             else:
                 pair, pair_rows = k.pair_plan(M, N, K, self.num_sms) if out.dtype == torch.bfloat16 else (0, 0)
                 bn = k.tile_width_for(M, N, self.num_sms)
-                if not pair and out.dtype == torch.bfloat16 and M <= 4 * self.split_rows:
+                # 128 x 128 tiles with the weights on the 128-row side, two CTAs an SM (see the kernel's dispatch):
+                tiles = -(-N // 128) * -(-M // 128)
+                if out.dtype == torch.bfloat16 and M <= 4 * self.split_rows and K >= N:
+                    # as many slices of the inner dimension as find a place, if these are three or more.  (Not where the
+                    # result is wider than the inner dimension: the rotary kernel behind q/k/v would rather read it
+                    # whole.)  Whole prompts at 1.8B sizes, one product at a time, ms: 400 tokens 3.12 -> 3.02 (output),
+                    # 3.03 (down), 700 tokens 3.48 -> 3.42 (down); two slices lose (1,000 tokens, output: 4.17 -> 4.24).
+                    slices = min(4, 2 * self.num_sms // tiles, K // 512)
+                    if slices >= 3:
+                        parts = self.ws.get("splitk_wide:" + tag, slices * M, N, torch.float32,
+                                            cap=16 * self.split_rows).view(slices, M, N)
+                        k.gemm_tcgen05(x, w, bias, parts, self.err, split_k=slices, swap=True, bn=128)
+                        self.launches += 1
+                        return Partials(parts)
+                # (pairs that would leave 40 % of the SMs idle give way: 7B sizes, 400 tokens, down: 7.90 -> 7.43 ms)
+                half_empty = pair and -(-M // pair_rows) * -(-N // pair) * 2 <= 0.6 * self.num_sms
+                if (not pair or half_empty) and out.dtype == torch.bfloat16 and M <= 4 * self.split_rows:
                     # A few hundred tokens and a long inner dimension (the down projection): 128 x 128
                     # tiles are too few for the SMs and re-read the operands too often.  Tiles of 128
                     # features x 256 tokens over slices of the inner dimension do better (measured
