@@ -77,13 +77,12 @@ class StepContext:
                                        # a token id <= -2 in ``tokens`` is read from row -id - 2
     graph_bucket: int = 0       # > 0: a decode step padded to this many entries
     real_entries: int = 0
-    graph_key: Optional[tuple] = None   # a step with prompt portions whose rows are padded to a
-                                        # multiple of 64 so that a captured graph fits it; the
+    graph_key: Optional[tuple] = None   # a step with prompt portions whose rows are padded to 16 or
+                                        # a multiple of 64 so that a captured graph fits it; the
                                         # padding rows have tok_entry -1 and belong to no entry,
                                         # padding entries have no rows and no cached length, and
                                         # the wanted rows beyond ``real_want`` repeat row 0
     real_want: int = 0
-    replay: bool = False        # a step with a graph_key: replay its graph (else launch its kernels)
     single_entries: int = 0     # > 0: a step with prompt portions whose entries of exactly one token
                                 # (decoded tokens, about this many) are worth a kernel of their own:
                                 # an attention mixer may give them to its split-KV decode kernel and
@@ -182,8 +181,6 @@ class ModelRunner:
         self._pad_with_copies = not mixer_state
         self.graph_replays = 0
         self.graph_captures = 0                    # steps that ran kernel by kernel and were recorded for their shape
-        self._step_done = torch.cuda.Event()       # recorded behind every step's kernels
-        self._step_done.record()
 
     # ---- cache geometry -------------------------------------------------
     def _build_cache(self) -> None:
@@ -327,7 +324,7 @@ class ModelRunner:
             if held.size > 1 and (pad_to or singles):
                 longest = int(held.max())
                 uneven = longest >= UNEVEN_KEYS and 2 * longest * held.size > 3 * int(held.sum())
-        # a small step with prompt portions: its rows are padded to a multiple of 64, its entries
+        # a small step with prompt portions: its rows are padded to 16 or a multiple of 64, its entries
         # and wanted places to a power of two, and from the second step of the same (rows,
         # entries, wanted, single-token entries) on a captured graph is replayed
         key = None
@@ -336,7 +333,10 @@ class ModelRunner:
         # small ones, which the host could not launch as fast as the device runs them, get one)
         limit = self.cfg.graph_max_tokens if n_entries <= 2 else self.cfg.graph_max_tokens // 4
         if (not pad_to and self._graphs_ok and 0 < n_tokens <= limit):
-            rows = min(-(-n_tokens // 64) * 64, self.cap_tokens)
+            # (few rows to 16: the products' tiles come that narrow; whole prompts of 8 tokens at 1.8B sizes 2.07 -> 1.61 ms,
+            # of 9 at 4B 2.86 -> 2.31, of 14 at 7B 3.96 -> 3.36, replayed where they had been launched one by one)
+            rows = 16 if n_tokens <= 16 else -(-n_tokens // 64) * 64
+            rows = min(rows, self.cap_tokens)
             wanted = sum(len(e.want) for e in entries)
             shape = ("rows", rows, self._power_of_two(n_entries, self.cap_entries),
                      self._power_of_two(wanted, rows) if wanted else 0,
@@ -397,15 +397,6 @@ class ModelRunner:
         ctx.short_prompts = short_prompts
         ctx.uneven = uneven
         ctx.all_single = int(cnt.max()) == 1
-        # While the device still runs the step before, the host launches this step's kernels
-        # behind it at no cost, and launched one by one they ran a little faster than replayed
-        # (a serving mix: 5 % per step): a graph pays when the device waits for the host.  The
-        # step is padded to its shape either way, so that both ways run the same kernels on the
-        # same rows and give the same bits.
-        # (A step of nothing but single tokens is a few hundred kernels of a few microseconds: the host
-        # cannot launch them as fast as the device runs them, busy or not, so its graph is always replayed.
-        # Measured at 295 kernels a step: 3.2 ms launched one by one against the device's own time.)
-        ctx.replay = key is not None and (int(cnt.max()) == 1 or self._step_done.query())
         ctx.real_want = n_want if key is None else real_want
         ctx.n_tokens, ctx.n_entries, ctx.n_want = n_tokens, n_entries, n_want
         # a padded step never counts as one of single tokens only: its filling entries have none
@@ -432,18 +423,18 @@ class ModelRunner:
         entries and of their ``want``."""
         ctx = self.prepare(entries, reserved)
         self.steps += 1
-        try:
-            if ctx.graph_bucket:
-                # (a graph holds the number of key slices its attention was recorded with: short
-                # contexts, which take fewer, have graphs of their own)
-                short = ctx.max_kv_len <= SHORT_CONTEXT
-                return self._replay(ctx, ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
-                                    + (UNEVEN_GRAPH_KEY if ctx.uneven else 0))[:ctx.real_entries]
-            if ctx.graph_key is not None and ctx.replay:
-                return self._replay(ctx, ctx.graph_key)[:ctx.real_want]
-            return self.model.forward(ctx, self.pools.layers)[:ctx.real_want]
-        finally:
-            self._step_done.record()
+        if ctx.graph_bucket:
+            # (a graph holds the number of key slices its attention was recorded with: short
+            # contexts, which take fewer, have graphs of their own)
+            short = ctx.max_kv_len <= SHORT_CONTEXT
+            return self._replay(ctx, ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
+                                + (UNEVEN_GRAPH_KEY if ctx.uneven else 0))[:ctx.real_entries]
+        if ctx.graph_key is not None:
+            # (always: the host cannot launch a few hundred kernels as fast as the device runs them, busy or
+            # not.  Whole prompts back to back, 1.8B sizes, launched one by one / replayed, ms: 100 tokens 2.65 / 2.02,
+            # 137 tokens 2.30 / 2.08, 250 tokens 2.67 / 2.21, 700 tokens 3.51 / 3.41, 2,048 tokens 7.16 / 7.11)
+            return self._replay(ctx, ctx.graph_key)[:ctx.real_want]
+        return self.model.forward(ctx, self.pools.layers)[:ctx.real_want]
 
     # ---- captured decode steps -----------------------------------------
     def _bucket(self, n: int) -> int:
