@@ -126,6 +126,7 @@ struct GemmParams {
     int* err;
     const uint8_t* prefetch;        // what the NEXT product of the step will stream (its weights), or null:
     long long prefetch_bytes;       // asked into L2 by this kernel's idle warp as soon as it starts
+    int slices;                     // of the inner dimension (the two-SM kernel; the others have them in their grid)
     int group_features, group_rows; // grouped activations (0: all features read the same rows)
 };
 // The first row of the activations that features from `feature` on read.
@@ -678,7 +679,9 @@ __device__ __forceinline__ void cluster_sync_all() {
 // A and BN / 2 rows of B per k-block for twice the products, the least operand traffic per product
 // of all the kernels here; with more than 256 accumulator columns per tile there is no second
 // accumulator to work into while the epilogue reads, so the epilogue of a tile is not hidden.
-template <int BN, int STAGES, bool SILU, int MT = 1>
+// PARTS: the inner dimension in p.slices slices, float partial sums of each (p.split_stride apart); a slice of a tile is
+// a unit of work of its own.
+template <int BN, int STAGES, bool SILU, int MT = 1, bool PARTS = false>
 __global__ void __launch_bounds__(NUM_THREADS)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const GemmParams p) {
@@ -706,8 +709,14 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
     constexpr int TILE_ROWS = 2 * BM * MT;
     const int tiles_a = (p.rows_a + TILE_ROWS - 1) / TILE_ROWS, tiles_b = (p.rows_b + BN - 1) / BN;
-    const int num_tiles = tiles_a * tiles_b;
-    const int num_kb = (p.k + BK - 1) / BK;
+    const int whole_tiles = tiles_a * tiles_b, num_tiles = PARTS ? whole_tiles * p.slices : whole_tiles;
+    const int all_kb = (p.k + BK - 1) / BK;
+    // k-blocks of a unit, dealt out to the slices as evenly as they go
+    auto kb_begin = [&](int tile) { return PARTS ? (int)((long long)(tile / whole_tiles) * all_kb / p.slices) : 0; };
+    auto kb_count = [&](int tile) {
+        return PARTS ? (int)((long long)(tile / whole_tiles + 1) * all_kb / p.slices) - kb_begin(tile) : all_kb;
+    };
+    auto place = [&](int tile) { return PARTS ? tile % whole_tiles : tile; };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -740,28 +749,29 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     if (warp == 0 && lane == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
         // (the weights depend on no earlier kernel: those of the first stages are asked for before the wait)
-        const int early = pair < num_tiles ? min(num_kb, STAGES) : 0;
+        const int early = pair < num_tiles ? min(kb_count(pair), STAGES) : 0;
         for (int kb = 0; kb < early; ++kb) {
             if (rank == 0) mbar_expect_tx(smem_u32(&full[kb]), 2 * (A_BYTES + B_BYTES));
-            tma_load_2d_pair(smem_u32(smem_b + kb * B_BYTES), &map_b, map_to_cta(smem_u32(&full[kb]), 0), kb * BK,
-                             pair / tiles_a * BN + (int)rank * BH);
+            tma_load_2d_pair(smem_u32(smem_b + kb * B_BYTES), &map_b, map_to_cta(smem_u32(&full[kb]), 0),
+                             (kb_begin(pair) + kb) * BK, place(pair) / tiles_a * BN + (int)rank * BH);
         }
         pdl_wait();
         int it = 0;
         for (int tile = pair; tile < num_tiles; tile += num_pairs) {
-            const int a0 = (tile % tiles_a) * TILE_ROWS + (int)rank * BM + group_row0(p, (tile / tiles_a) * BN);
-            const int b0 = (tile / tiles_a) * BN + (int)rank * BH;
+            const int at = place(tile), kb0 = kb_begin(tile), num_kb = kb_count(tile);
+            const int a0 = (at % tiles_a) * TILE_ROWS + (int)rank * BM + group_row0(p, (at / tiles_a) * BN);
+            const int b0 = (at / tiles_a) * BN + (int)rank * BH;
             for (int kb = 0; kb < num_kb; ++kb, ++it) {
                 const int s = it % STAGES;
                 const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
                 if (it >= early) {
                     if (!mbar_wait(smem_u32(&empty[s]), ((it / STAGES) & 1) ^ 1, abort_flag)) goto done;
                     if (rank == 0) mbar_expect_tx(smem_u32(&full[s]), 2 * (A_BYTES + B_BYTES));   // both CTAs' bytes
-                    tma_load_2d_pair(smem_u32(smem_b + s * B_BYTES), &map_b, bar, kb * BK, b0);
+                    tma_load_2d_pair(smem_u32(smem_b + s * B_BYTES), &map_b, bar, (kb0 + kb) * BK, b0);
                 }
 #pragma unroll
                 for (int m = 0; m < MT; ++m)
-                    tma_load_2d_pair(smem_u32(smem_a + s * A_BYTES + m * A_SUB), &map_a, bar, kb * BK,
+                    tma_load_2d_pair(smem_u32(smem_a + s * A_BYTES + m * A_SUB), &map_a, bar, (kb0 + kb) * BK,
                                      a0 + m * 2 * BM);
             }
         }
@@ -775,6 +785,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
             if (!mbar_wait(smem_u32(&acc_empty[acc]), ((local / NACC) & 1) ^ 1, abort_flag)) goto done;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tmem_d = tmem_base + (uint32_t)(acc * MT * BN);
+            const int num_kb = kb_count(tile);
             for (int kb = 0; kb < num_kb; ++kb, ++it) {
                 const int s = it % STAGES;
                 if (!mbar_wait(smem_u32(&full[s]), (it / STAGES) & 1, abort_flag)) goto done;
@@ -799,7 +810,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         int local = 0;
         for (int tile = pair; tile < num_tiles; tile += num_pairs, ++local) {
             const int acc = local % NACC;
-            const int a0 = (tile % tiles_a) * TILE_ROWS + (int)rank * BM, b0 = (tile / tiles_a) * BN;
+            const int at = place(tile), a0 = (at % tiles_a) * TILE_ROWS + (int)rank * BM, b0 = (at / tiles_a) * BN;
+            GemmParams to = p;
+            if (PARTS) to.out = (float*)p.out + (long long)(tile / whole_tiles) * p.split_stride;
             if (!mbar_wait(smem_u32(&acc_full[acc]), (local / NACC) & 1, abort_flag)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t trow = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * MT * BN);
@@ -813,7 +826,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 if (a >= p.rows_a) continue;
                 const int b_first = b0 + c0;
                 if (b_first >= p.rows_b) continue;
-                store_chunk32<false, SILU>(p, r, a, b_first);
+                store_chunk32<PARTS, SILU>(to, r, a, b_first);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -927,12 +940,12 @@ int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const GemmPa
     return crane_launch(kern, dim3(ctas), dim3(NUM_THREADS), smem, st, ma, mb, p);
 }
 
-template <int BN, int STAGES, bool SILU, int MT = 1>
+template <int BN, int STAGES, bool SILU, int MT = 1, bool PARTS = false>
 int launch_pair(const void* A, const void* B, int rows_a, int rows_b, int k, long long lda, long long ldb,
                 const GemmParams& p, int map_rows_a, cudaStream_t st) {
     constexpr size_t smem = STAGES * (MT * BM * BK * 2 + (BN / 2) * BK * 2) + (2 * STAGES + 4) * 8 + 16 + 1024;
     static_assert(smem <= 232448, "more shared memory than a CTA can have");
-    auto kern = gemm_bf16_pair_kernel<BN, STAGES, SILU, MT>;
+    auto kern = gemm_bf16_pair_kernel<BN, STAGES, SILU, MT, PARTS>;
     static bool configured = false;
     static int sms = 0;
     if (!configured) {
@@ -946,7 +959,7 @@ int launch_pair(const void* A, const void* B, int rows_a, int rows_b, int k, lon
     CUtensorMap ma, mb;
     if (!make_map(&ma, A, map_rows_a, k, lda, BM) || !make_map(&mb, B, rows_b, k, ldb, BN / 2))
         return (int)cudaErrorInvalidValue;
-    const int tiles = ((rows_a + 2 * BM * MT - 1) / (2 * BM * MT)) * ((rows_b + BN - 1) / BN);
+    const int tiles = ((rows_a + 2 * BM * MT - 1) / (2 * BM * MT)) * ((rows_b + BN - 1) / BN) * (PARTS ? p.slices : 1);
     const int pairs = tiles < sms / 2 ? tiles : sms / 2;
     return crane_launch_cluster(kern, dim3(2 * pairs), dim3(NUM_THREADS), smem, dim3(2, 1, 1), st, ma, mb, p);
 }
@@ -1006,7 +1019,7 @@ CRANE_API int crane_gemm_bf16_tcgen05(const void* A, const void* B, const float*
     if (split_k > num_kb) split_k = num_kb;
     GemmParams p;
     p.rows_a = rows_a; p.rows_b = rows_b; p.k = k;
-    p.out = out; p.ld_out = ld_out; p.split_stride = split_stride; p.bias = bias; p.err = err;
+    p.out = out; p.ld_out = ld_out; p.split_stride = split_stride; p.slices = 1; p.bias = bias; p.err = err;
     p.group_features = group_features; p.group_rows = group_rows;
     p.prefetch = ((uintptr_t)prefetch & 15) ? nullptr : (const uint8_t*)prefetch;   // (only the narrow-tile kernel asks)
     p.prefetch_bytes = prefetch_bytes > 0 ? prefetch_bytes : 0;
@@ -1066,7 +1079,7 @@ CRANE_API int crane_gemm_bf16_tcgen05(const void* A, const void* B, const float*
 CRANE_API int crane_gemm_bf16_pair(const void* A, const void* B, const float* bias, void* out, int rows_a,
                                    int rows_b, int k, long long lda, long long ldb, long long ld_out,
                                    int bn, int tile_rows, int epilogue, int group_features, int group_rows,
-                                   int* err, cudaStream_t st) {
+                                   int slices, long long split_stride, int* err, cudaStream_t st) {
     if (rows_a <= 0 || rows_b <= 0) return 0;
     if (k <= 0 || (k & 7) || (lda & 7) || (ldb & 7) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15))
         return (int)cudaErrorInvalidValue;
@@ -1074,9 +1087,15 @@ CRANE_API int crane_gemm_bf16_pair(const void* A, const void* B, const float* bi
     const bool tall = tile_rows == 4 * BM;                  // 512-row tiles: bn 192, 224 or 256
     GemmParams p;
     p.rows_a = rows_a; p.rows_b = rows_b; p.k = k;
-    p.out = out; p.ld_out = ld_out; p.split_stride = 0; p.bias = bias; p.err = err;
+    p.out = out; p.ld_out = ld_out; p.split_stride = split_stride; p.slices = slices; p.bias = bias; p.err = err;
     p.prefetch = nullptr; p.prefetch_bytes = 0;
     p.group_features = group_features; p.group_rows = group_rows;
+    if (slices > 1) {
+        // float partial sums [slices][rows_a][ld_out]
+        if (bias != nullptr || epilogue != 0 || group_features > 0 || tall || bn != 256 || slices > (k + BK - 1) / BK)
+            return (int)cudaErrorInvalidValue;
+        return launch_pair<256, 6, false, 1, true>(A, B, rows_a, rows_b, k, lda, ldb, p, rows_a, st);
+    }
     int map_rows = rows_a;
     if (group_features > 0) {
         if (group_features % bn || group_rows < rows_a || epilogue != 0) return (int)cudaErrorInvalidValue;

@@ -28,7 +28,7 @@ _SIGNATURES = {
     "crane_sum_parts": [P, I, L, L, P, L, I, I, P],
     "crane_gemm_simt": [I, I, P, P, P, P, I, I, I, L, L, L, P],
     "crane_gemm_bf16_tcgen05": [P, P, P, P, I, I, I, L, L, L, I, I, I, I, I, L, I, I, I, P, L, P, P],
-    "crane_gemm_bf16_pair": [P, P, P, P, I, I, I, L, L, L, I, I, I, I, I, P, P],
+    "crane_gemm_bf16_pair": [P, P, P, P, I, I, I, L, L, L, I, I, I, I, I, I, L, P, P],
     "crane_paged_attention_simt": [I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P, P, P],
     "crane_paged_decode_attention_supports": [I, I, I],
     "crane_paged_decode_attention": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, P, P, P, I, L, I, I, I, P, I, I, P, P],
@@ -782,20 +782,24 @@ class Kernels:
     PAIR_TILES = (256, 224, 192, 128)
 
     def gemm_pair(self, x, w, bias, out, err, bn: int = 256, silu_mul: bool = False,
-                  tile_rows: int = 256, group_features: int = 0, group_rows: int = 0) -> None:
+                  tile_rows: int = 256, group_features: int = 0, group_rows: int = 0, split_k: int = 1) -> None:
         """out[M,N] (bf16) = x[M,K] @ w[N,K]^T (+ bias) for many tokens, every
         256 x ``bn`` tile computed by two SMs together (tcgen05 cta_group::2).
         ``silu_mul`` as in ``gemm_tcgen05``.  ``tile_rows`` 512: tiles of 512
         tokens x ``bn`` (192, 224 or 256) features, two accumulators per SM.
-        ``group_features`` as in ``gemm_tcgen05``."""
+        ``group_features`` as in ``gemm_tcgen05``.  ``split_k`` > 1: ``out`` is float [slices, M, N] of
+        partial sums (tiles of 256 x 256, no bias)."""
         M, K = x.shape
         N = w.shape[0]
-        assert out.dtype == torch.bfloat16 and out.stride(1) == 1 and bn in self.PAIR_TILES
-        assert tuple(out.shape) == ((M, N // 2) if silu_mul else (M, N))
+        assert out.stride(-1) == 1 and bn in self.PAIR_TILES
+        if split_k > 1:
+            assert out.dtype == torch.float32 and tuple(out.shape) == (split_k, M, N) and not silu_mul and bias is None
+        else:
+            assert out.dtype == torch.bfloat16 and tuple(out.shape) == ((M, N // 2) if silu_mul else (M, N))
         self._check(self.lib.crane_gemm_bf16_pair(
             x.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K, x.stride(0), w.stride(0),
-            out.stride(0), bn, tile_rows, 1 if silu_mul else 0, int(group_features), int(group_rows),
-            err.data_ptr(), self._stream(x)), "gemm_pair")
+            out.stride(-2), bn, tile_rows, 1 if silu_mul else 0, int(group_features), int(group_rows),
+            int(split_k), out.stride(0) if split_k > 1 else 0, err.data_ptr(), self._stream(x)), "gemm_pair")
 
     WIDE_TILES = (256, 224, 192, 160, 128)
 

@@ -259,6 +259,18 @@ class Runtime:
             else:
                 pair, pair_rows = k.pair_plan(M, N, K, self.num_sms) if out.dtype == torch.bfloat16 else (0, 0)
                 bn = k.tile_width_for(M, N, self.num_sms)
+                # Large products of few tiles: 256 x 256 tiles on pairs of SMs, which load the least, in slices of the inner
+                # dimension that fill one round.  Whole prompts, down projection: 7B sizes, 300 tokens 6.64 -> 6.36 ms, 400
+                # tokens 8.12 -> 7.20; at 1.8B sizes (less than the 30 GFLOP below) it loses to the smaller tiles.
+                slices = self.num_sms // 2 // (-(-M // 256) * -(-N // 256))
+                if (slices >= 2 and out.dtype == torch.bfloat16 and bias is None and M <= 4 * self.split_rows
+                        and K >= N and 2.0 * M * N * K >= 3e10 and K // slices >= 2048):
+                    slices = min(slices, 4)
+                    parts = self.ws.get("splitk_wide:" + tag, slices * M, N, torch.float32,
+                                        cap=16 * self.split_rows).view(slices, M, N)
+                    k.gemm_pair(x, w, None, parts, self.err, split_k=slices)
+                    self.launches += 1
+                    return Partials(parts)
                 # 128 x 128 tiles with the weights on the 128-row side, two CTAs an SM (see the kernel's dispatch):
                 tiles = -(-N // 128) * -(-M // 128)
                 if out.dtype == torch.bfloat16 and M <= 4 * self.split_rows and K >= N:
@@ -273,9 +285,7 @@ class Runtime:
                         k.gemm_tcgen05(x, w, bias, parts, self.err, split_k=slices, swap=True, bn=128)
                         self.launches += 1
                         return Partials(parts)
-                # (pairs that would leave 40 % of the SMs idle give way: 7B sizes, 400 tokens, down: 7.90 -> 7.43 ms)
-                half_empty = pair and -(-M // pair_rows) * -(-N // pair) * 2 <= 0.6 * self.num_sms
-                if (not pair or half_empty) and out.dtype == torch.bfloat16 and M <= 4 * self.split_rows:
+                if not pair and out.dtype == torch.bfloat16 and M <= 4 * self.split_rows:
                     # A few hundred tokens and a long inner dimension (the down projection): 128 x 128
                     # tiles are too few for the SMs and re-read the operands too often.  Tiles of 128
                     # features x 256 tokens over slices of the inner dimension do better (measured

@@ -1175,3 +1175,18 @@ def test_add_rmsnorm_many_rows(K, dtype, n, hidden, parts):
     d = want_x.double()
     want = d * torch.rsqrt((d * d).mean(-1, keepdim=True) + 1e-5) * w.double()
     assert rel_err(out, want) < TOL[dtype]
+
+
+# one and several rounds of units over the pairs of SMs, slices that do not divide the k-blocks, rows and columns past the last tile
+@pytest.mark.parametrize("M,N,K_,slices", [(448, 512, 768, 2), (300, 2048, 2056, 4), (704, 3080, 1032, 3), (1024, 4096, 640, 5)])
+def test_gemm_pair_slices(K, err, M, N, K_, slices):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(M)
+    a, w = (torch.randn(r, K_, generator=g, device=DEV).bfloat16() for r in (M, N))
+    parts = torch.full((slices + 1, M, N), 7.0, device=DEV)
+    K.gemm_pair(a, w, None, parts[:slices], err, split_k=slices)
+    assert int(err.item()) == 0 and bool((parts[slices] == 7.0).all())
+    blocks = (K_ + 63) // 64
+    for s in range(slices):
+        lo, hi = s * blocks // slices * 64, min(K_, (s + 1) * blocks // slices * 64)
+        assert rel_err(parts[s], a[:, lo:hi].double() @ w[:, lo:hi].double().T) < acc_tol(hi - lo)
