@@ -72,11 +72,11 @@ gemm_nt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* 
 }
 
 // ---- float operands, rows of whole 16-byte pieces --------------------------------------------------
-// What bounds it: with few rows the weights' way from DRAM; with many the way of the operands from shared memory
-// into registers (16 bytes a lane take four clocks of an SM, whether or not the lanes read the same
-// ones), and behind it the FP32 cores.  A whole prompt of 97 tokens at hidden 2048, inner 6144, 32 layers:
-// 39.3 -> 22.2 ms, gate and up 245 us a layer; the kernel below, which reads every operand 4 bytes at a
-// time and has 32 to 384 CTAs without slices, was the whole difference.
+// What bounds it: with few rows the weights' way from DRAM; with many the operands' way from shared memory
+// into registers (16 bytes a lane take four clocks of an SM, whether or not the lanes read the same ones), and
+// behind it the FP32 cores.  Whole prompts at hidden 2048, inner 6144, 32 layers, 32-bit: 97 tokens 39.3 -> 22.2 ms
+// (17.0 with the slices below and wider loads in the attention), 24 tokens 34.5 -> 6.1 ms; `gemm_nt_kernel`, which
+// reads every operand 4 bytes at a time and has no slices, took nearly all of it before.
 //
 // A CTA computes BM x BN results over a slice of the inner dimension, which a cluster of up to 8 CTAs
 // shares (the products of a step of 97 tokens have 16 to 96 tiles for 148 SMs); the slices' sums are
