@@ -83,6 +83,7 @@ class StepContext:
                                         # padding entries have no rows and no cached length, and
                                         # the wanted rows beyond ``real_want`` repeat row 0
     real_want: int = 0
+    replay: bool = False        # a step with a graph_key: replay its graph, or capture one (else launch its kernels)
     single_entries: int = 0     # > 0: a step with prompt portions whose entries of exactly one token
                                 # (decoded tokens, about this many) are worth a kernel of their own:
                                 # an attention mixer may give them to its split-KV decode kernel and
@@ -180,6 +181,8 @@ class ModelRunner:
                                   if any(f.kind == "state" for f in mx.cache_need().flat()))
         self._pad_with_copies = not mixer_state
         self.graph_replays = 0
+        self._step_done = torch.cuda.Event()       # recorded behind every step's kernels
+        self._step_done.record()
         self.graph_captures = 0                    # steps that ran kernel by kernel and were recorded for their shape
 
     # ---- cache geometry -------------------------------------------------
@@ -397,6 +400,14 @@ class ModelRunner:
         ctx.short_prompts = short_prompts
         ctx.uneven = uneven
         ctx.all_single = int(cnt.max()) == 1
+        # The host cannot launch a few hundred kernels as fast as the device runs them, busy or not, so a graph that is
+        # there is always replayed (whole prompts back to back, 1.8B sizes, launched one by one / replayed, ms: 100 tokens
+        # 2.65 / 2.02, 137 tokens 2.30 / 2.08, 250 tokens 2.67 / 2.21, 700 tokens 3.51 / 3.41, 2,048 tokens 7.16 / 7.11).  A
+        # capture costs tens of milliseconds, so while the device is busy a shape has to come often to get one (a
+        # prompt of 8,192 tokens in four portions on a new engine, 7B sizes: 110 ms, 143 with a capture in it).  Both
+        # ways run the same kernels on the same rows and give the same bits.
+        ctx.replay = key is not None and (self._has_graph(key) or int(cnt.max()) == 1 or seen >= self.CAPTURE_BUSY
+                                          or self._step_done.query())
         ctx.real_want = n_want if key is None else real_want
         ctx.n_tokens, ctx.n_entries, ctx.n_want = n_tokens, n_entries, n_want
         # a padded step never counts as one of single tokens only: its filling entries have none
@@ -423,18 +434,18 @@ class ModelRunner:
         entries and of their ``want``."""
         ctx = self.prepare(entries, reserved)
         self.steps += 1
-        if ctx.graph_bucket:
-            # (a graph holds the number of key slices its attention was recorded with: short
-            # contexts, which take fewer, have graphs of their own)
-            short = ctx.max_kv_len <= SHORT_CONTEXT
-            return self._replay(ctx, ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
-                                + (UNEVEN_GRAPH_KEY if ctx.uneven else 0))[:ctx.real_entries]
-        if ctx.graph_key is not None:
-            # (always: the host cannot launch a few hundred kernels as fast as the device runs them, busy or
-            # not.  Whole prompts back to back, 1.8B sizes, launched one by one / replayed, ms: 100 tokens 2.65 / 2.02,
-            # 137 tokens 2.30 / 2.08, 250 tokens 2.67 / 2.21, 700 tokens 3.51 / 3.41, 2,048 tokens 7.16 / 7.11)
-            return self._replay(ctx, ctx.graph_key)[:ctx.real_want]
-        return self.model.forward(ctx, self.pools.layers)[:ctx.real_want]
+        try:
+            if ctx.graph_bucket:
+                # (a graph holds the number of key slices its attention was recorded with: short
+                # contexts, which take fewer, have graphs of their own)
+                short = ctx.max_kv_len <= SHORT_CONTEXT
+                return self._replay(ctx, ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
+                                    + (UNEVEN_GRAPH_KEY if ctx.uneven else 0))[:ctx.real_entries]
+            if ctx.graph_key is not None and ctx.replay:
+                return self._replay(ctx, ctx.graph_key)[:ctx.real_want]
+            return self.model.forward(ctx, self.pools.layers)[:ctx.real_want]
+        finally:
+            self._step_done.record()
 
     # ---- captured decode steps -----------------------------------------
     def _bucket(self, n: int) -> int:
@@ -452,6 +463,11 @@ class ModelRunner:
             step = max(4, b // 16)
             b = -(-n // step) * step
         return min(b, self.cap_entries)
+
+    CAPTURE_BUSY = 16           # a shape that has come so often is captured while the device is busy, too
+
+    def _has_graph(self, key) -> bool:
+        return key in self._graphs and self._graph_generation == self.rt.ws.generation
 
     MAX_SHAPE_GRAPHS = 256      # graphs of small steps kept; the least recently used one goes first
 
