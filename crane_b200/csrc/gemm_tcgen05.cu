@@ -731,6 +731,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    // The peer has to be running before either CTA asks for the pair's tensor memory: the CTAs of a cluster begin up to
+    // a microsecond apart where the SMs come free one by one, and a pair whose first CTA asked 0.7 us before its
+    // second one had begun never got an answer, with all tensor memory of both SMs free.  (The peer's barriers exist
+    // from here on, too.  Its own tensor memory it has before its copies, which every product waits for.)
+    cluster_sync_all();
     if (warp == 1) {
         // the same warp of both CTAs, the same slot offset
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -741,7 +746,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    cluster_sync_all();                          // the peer's barriers exist before anything signals them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();

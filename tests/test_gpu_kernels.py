@@ -1190,3 +1190,37 @@ def test_gemm_pair_slices(K, err, M, N, K_, slices):
     for s in range(slices):
         lo, hi = s * blocks // slices * 64, min(K_, (s + 1) * blocks // slices * 64)
         assert rel_err(parts[s], a[:, lo:hi].double() @ w[:, lo:hi].double().T) < acc_tol(hi - lo)
+
+
+def test_gemm_pair_behind_kernels_that_end_raggedly(K, err):
+    """The sequence of a parallel block's feed-forward (a product on single SMs, the activation with many small CTAs, a
+    product on pairs of SMs in slices, the norm), launched ahead of each other's end and replayed without gaps: the two CTAs
+    of a pair begin at different times there.  Every replay ends, with the same bits."""
+    M, N, K_ = 832, 2048, 9216
+    g = torch.Generator(device=DEV)
+    g.manual_seed(1)
+    h, up_w, down_w = (torch.randn(*s, generator=g, device=DEV).mul_(0.05).bfloat16() for s in ((M, N), (K_, N), (N, K_)))
+    up, act = (torch.empty(M, K_, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    parts, normed = torch.empty(2, M, N, device=DEV), torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+    x, pq, w = torch.zeros(M, N, device=DEV), torch.tensor([0.3, 0.7], device=DEV), torch.ones(N, device=DEV)
+    from crane_b200.kernels import Partials
+
+    def layer():
+        K.gemm_tcgen05(h, up_w, None, up, err, bn=224)
+        K.xielu(up, act, pq)
+        K.gemm_pair(act, down_w, None, parts, err, split_k=2)
+        K.add_rmsnorm(x, Partials(parts), w, 1e-5, normed)
+    layer()
+    torch.cuda.synchronize()
+    first = parts.clone()
+    assert rel_err(first.sum(0), act.double() @ down_w.double().T) < acc_tol(K_)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(8):
+            layer()
+    for _ in range(50):
+        parts.fill_(7.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(parts, first)
+    assert int(err.item()) == 0
