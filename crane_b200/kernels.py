@@ -779,6 +779,32 @@ class Kernels:
                 best, best_eff = s, eff
         return best
 
+    @staticmethod
+    def few_rows_tile(m: int) -> int:
+        return 16 if m <= 16 else 32 if m <= 32 else 64 if m <= 64 else 128 if m <= 128 else 256
+
+    @classmethod
+    def few_rows_plan(cls, m: int, n: int, k: int, sms: int):
+        """(tokens of a tile, slices of the inner dimension) of a product of at most 256 tokens, whose weight rows fill the
+        MMA's 128-wide side and whose inner dimension is cut until every SM has a tile to stream."""
+        bn, tiles, row_tiles = cls.few_rows_tile(m), -(-n // 128), -(-m // 64)
+        most = 2 * sms // (tiles * row_tiles)
+        if bn == 256 and most >= 1 and (most >= 3 or k // most <= 4096):
+            # More than 128 tokens: tiles of 64, two CTAs an SM, fewer slices of the inner dimension, instead of
+            # one tile of 256 (padded) tokens that takes an SM for itself and leaves up to 8 partial sums of
+            # everything.  Where all tiles are there at once (else the weights came from DRAM once per tile of
+            # tokens) and a CTA's share of the inner dimension is not long.  Whole prompts, ms: 1.8B sizes, 137
+            # tokens 2.41 -> 2.08, 250 tokens 2.68 -> 2.21; 7B sizes, 250 tokens, down with 2 slices of 7,168
+            # 5.01 -> 5.16, hence the second condition.
+            return 64, min(8, most, max(1, k // 256))
+        # at most 8: the consumers of partial sums fetch eight slices at a time
+        return bn, min(cls.slices_for(tiles, k, sms), 8)
+
+    @classmethod
+    def few_rows_most_slices(cls, n: int, k: int, sms: int) -> int:
+        """The most slices that ``few_rows_plan`` gives any number of tokens (it changes with the kind of tile alone)."""
+        return max(cls.few_rows_plan(m, n, k, sms)[1] for m in (1, 129, 193))
+
     PAIR_TILES = (256, 224, 192, 128)
 
     def gemm_pair(self, x, w, bias, out, err, bn: int = 256, silu_mul: bool = False,

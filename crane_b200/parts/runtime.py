@@ -185,7 +185,7 @@ class Runtime:
                 k.lib.crane_set_pdl(0)
             try:
                 if M <= self.split_rows:
-                    k.gemm_tcgen05(x, wg, None, og, self.err, swap=True, bn=self._few_rows_tile(M))
+                    k.gemm_tcgen05(x, wg, None, og, self.err, swap=True, bn=k.few_rows_tile(M))
                 else:
                     k.gemm_tcgen05(x, wg, None, og, self.err, bn=128)
             finally:
@@ -194,10 +194,6 @@ class Runtime:
             self.launches += 1
             self._after_product = self.launches
         return out
-
-    @staticmethod
-    def _few_rows_tile(M: int) -> int:
-        return 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
 
     def _linear_bf16(self, x, w, bias, out, hint_next: bool = True, own_parts: Optional[str] = None,
                      group=None, keep_parts: bool = False) -> Act:
@@ -209,24 +205,7 @@ class Runtime:
         grp = {} if group is None else {"group_features": group[0], "group_rows": group[1]}
         if self.use_tcgen05 and k.tcgen05_takes(x, w):
             if M <= self.split_rows:
-                # few tokens: the weight rows fill the MMA's 128-wide side (the tokens its 16 to
-                # 256 wide side), and the inner dimension is cut into slices until every SM has a
-                # tile to stream
-                bn = self._few_rows_tile(M)
-                tiles = (N + 127) // 128
-                # at most 8: the consumers of partial sums fetch eight slices at a time
-                slices = min(k.slices_for(tiles, K, self.num_sms), 8)
-                most = 2 * self.num_sms // (tiles * -(-M // 64))
-                if bn == 256 and most >= 1 and (most >= 3 or K // most <= 4096):
-                    # More than 128 tokens: tiles of 64, two CTAs an SM, fewer slices of the inner dimension, instead of
-                    # one tile of 256 (padded) tokens that takes an SM for itself and leaves up to 8 partial sums of
-                    # everything.  Where all tiles are there at once (else the weights came from DRAM once per tile of
-                    # tokens) and a CTA's share of the inner dimension is not long.  Whole prompts, ms: 1.8B sizes, 137
-                    # tokens 2.41 -> 2.08, 250 tokens 2.68 -> 2.21; 7B sizes, 250 tokens, down with 2 slices of 7,168
-                    # 5.01 -> 5.16, hence the second condition.
-                    bn = 64
-                    tiles *= -(-M // 64)
-                    slices = min(8, most, max(1, K // 256))
+                bn, slices = k.few_rows_plan(M, N, K, self.num_sms)
                 nxt = self._next_weights(w) if w.is_contiguous() else None
                 # Measured in whole decode steps (Hunyuan-1.8B sizes): a single token gains 2.4 % at a
                 # context of 2,048 and 4.6 % at 8,192; from two tokens on the hints cost 1 to 4 % (the
@@ -235,8 +214,10 @@ class Runtime:
                 if not hint_next or M != 1:
                     nxt = None
                 if slices > 1:
-                    parts = self.ws.get("splitk:" + tag, slices * self.split_rows, N,
-                                        torch.float32, cap=slices * self.split_rows)
+                    # (a buffer that grew would throw the captured graphs away: it is made for the most slices
+                    # that any number of tokens takes)
+                    parts = self.ws.get("splitk:" + tag, slices * self.split_rows, N, torch.float32,
+                                        cap=k.few_rows_most_slices(N, K, self.num_sms) * self.split_rows)
                     parts = parts[:slices * M].view(slices, M, N)
                     k.gemm_tcgen05(x, w, bias, parts, self.err, split_k=slices, swap=True, bn=bn, prefetch=nxt, **grp)
                     self.launches += 1

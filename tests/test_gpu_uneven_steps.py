@@ -1,0 +1,131 @@
+"""Steps whose requests differ much in length, through the runner: the decode attention gives long contexts more key
+slices there, in graphs of their own where that is another kernel.  Decode and mixed steps with and without graphs, step
+after step as lengths change and as the batch flips between uneven and even, against the plain implementation; and
+that buffers stay where they are and no graph is captured that is not needed."""
+import numpy as np
+import pytest
+import torch
+
+import plain_hunyuan as ph
+import tiny_configs
+import trace_tools as tt
+
+pytestmark = pytest.mark.gpu
+
+# 8 key/value heads of 128: from 9 requests on (a bucket of 16) two key slices each, more for long contexts among short ones
+CFG = dict(tiny_configs.A, vocab_size=301, hidden_size=256, intermediate_size=384, num_attention_heads=16,
+           num_key_value_heads=8, head_dim=128, max_position_embeddings=2048)
+SHORT, LONG = [20, 33, 60, 5, 47, 28, 31, 52, 16, 40], [900, 700, 600]
+
+
+class Run:
+    """A runner, and for every request its tokens and the plain logits of all its places."""
+
+    def __init__(self, monkeypatch, folder, seqs=(), plain=(), **opts):
+        from crane_b200.generation import ModelForCausalLM
+        opts = dict(dict(page_size=64, num_pages=200, max_concurrent=32, max_batched_tokens=1024, chunk_size=1024), **opts)
+        self.model = ModelForCausalLM.from_pretrained(folder, "bf16", **opts)
+        self.r, self.seqs, self.plain = self.model.runner, seqs, plain
+        self.at = {i: 0 for i in range(len(seqs))}
+        self.balanced = {"fused": 0, "plain": 0}
+        k = self.r.rt.kernels
+        for kind, name in (("fused", "paged_decode_attention_fused"), ("plain", "paged_decode_attention")):
+            monkeypatch.setattr(k, name, self._counted(getattr(k, name), kind))
+
+    def _counted(self, inner, kind):
+        def call(*a, **kw):
+            self.balanced[kind] += kw.get("balance") is not None
+            return inner(*a, **kw)
+        return call
+
+    def step(self, counts, check=True):
+        """counts: {request: tokens of it}; the logits of every request's last place."""
+        from crane_b200.engine import StepEntry
+        entries = []
+        for i, n in counts.items():
+            entries.append(StepEntry(i, self.seqs[i][self.at[i]:self.at[i] + n], [n - 1]))
+            self.at[i] += n
+        got = self.r.step(entries)
+        if check:
+            self.compare(got, [(i, self.at[i] - 1) for i in counts])
+        return got
+
+    def compare(self, got, places):
+        want = np.stack([self.plain[i][p] for i, p in places])
+        got = got.float().cpu().numpy()
+        assert got.shape == want.shape and np.isfinite(got).all()
+        worst = np.abs(got - want).max(axis=1) / np.abs(want).max()
+        assert worst.max() < tt.TOL["bfloat16"], (places[int(worst.argmax())], worst.max())
+
+    def prefill(self, who, lens):
+        small = {i: n for i, n in zip(who, lens) if n < 100}
+        for i, n in zip(who, lens):
+            if n >= 100:
+                self.step({i: n})
+        if small:
+            self.step(small)
+
+    def done(self):
+        self.r.rt.check_errors()
+        for i, n in self.at.items():
+            if n:
+                self.r.end(i)
+        self.r.table.check()
+
+
+@pytest.fixture(scope="module")
+def uneven_model(tmp_path_factory):
+    from crane_b200.weights.random_init import write_model_folder
+    folder = write_model_folder(str(tmp_path_factory.mktemp("uneven")), CFG, 3, "bfloat16", std=0.05, norm_std=0.05)
+    return make(folder, 24)
+
+
+def make(folder, n):
+    cfg, w = ph.load_folder(folder)
+    rng = np.random.default_rng(5)
+    seqs = [rng.integers(0, cfg.vocab_size, 1000 if i >= len(SHORT) - 2 else 120).tolist() for i in range(n)]
+    plain = [ph.logits_all(cfg, w, s) for s in seqs]
+    return folder, seqs, plain
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_uneven_steps_match_the_plain_logits(uneven_model, monkeypatch, graphs):
+    run = Run(monkeypatch, *uneven_model, use_cuda_graphs=graphs)
+    short, long_ = list(range(10)), [10, 11, 12]
+    run.prefill(short + long_, SHORT + LONG)
+    every = {i: 1 for i in short + long_}
+    for _ in range(3):
+        run.step(every)                                     # 13 requests, uneven
+    assert run.balanced["fused"] > 0
+    for _ in range(3):
+        run.step({i: 1 for i in short})                     # 10 requests of the same bucket, even
+    for _ in range(2):
+        run.step(every)
+    run.step({9: 600})                                      # a short one grows: the lengths change under the graph
+    for _ in range(2):
+        run.step(every)
+    for t in range(4):                                      # beside a prompt, which ends with the step
+        run.step({**every, 13 + t: 30 + t})
+        run.r.end(13 + t)
+        run.at[13 + t] = 0
+    assert run.balanced["plain"] > 0
+    for _ in range(2):
+        run.step({i: 1 for i in [8, 9] + long_ + short[:6]})     # another composition of the bucket
+    assert (run.r.graph_replays > 0) == graphs
+    run.done()
+
+
+def test_buffers_stay_where_they_are(model_folders, monkeypatch):
+    """Steps of changing size at model layer sizes: a buffer that grows would throw all graphs away."""
+    from crane_b200.engine import StepEntry
+    run = Run(monkeypatch, model_folders("S18", "bfloat16"), max_concurrent=20)
+    r, rng = run.r, np.random.default_rng(1)
+    draw = lambda n: rng.integers(0, 1000, n).tolist()      # noqa: E731
+    for i, n in enumerate((250, 137, 192, 193, 40, 300, 700)):
+        r.step([StepEntry(i, draw(n), [n - 1])])
+    assert r.rt.ws.generation == 0
+    r.step([StepEntry(0, draw(1), [0])])
+    assert r.rt.ws.generation == 0 and len(r._graphs) >= 1
+    run.done()
+    for i in range(7):
+        r.end(i)

@@ -97,3 +97,16 @@ def test_query_tiles_exact_and_bound():
     for lens in ([320, 0, 0, 0], [1, 1, 1, 317], [127, 129, 63, 1], [80, 80, 80, 80]):
         exact = sum(-(-q // 128) for q in lens)
         assert exact <= query_tiles(c, 128)
+
+
+def test_few_rows_plan_and_its_bound():
+    """Products of at most 256 tokens: the buffer of their partial sums is made for the most slices that any number of
+    tokens takes, so that it never grows (which would throw captured graphs away)."""
+    for n in (128, 320, 2048, 3072, 4096, 6144, 12288, 28672, 120818):
+        for k in (64, 256, 2048, 4096, 14336):
+            plans = [Kernels.few_rows_plan(m, n, k, SMS) for m in range(1, 257)]
+            assert all(bn in (16, 32, 64, 128, 256) and 1 <= s <= 8 for bn, s in plans)
+            assert max(s for _, s in plans) == Kernels.few_rows_most_slices(n, k, SMS)
+    # one size, three numbers of slices: what a buffer made for the first caller would not hold
+    assert [Kernels.few_rows_plan(m, 2048, 2048, SMS) for m in (1, 137, 250)] == [(16, 8), (64, 6), (64, 4)]
+    assert Kernels.few_rows_plan(250, 4096, 14336, SMS) == (256, 8)        # a long share of the inner dimension: one tile of tokens
