@@ -145,6 +145,12 @@ class GqaAttention(Part):
             return CacheNeed("none")
         return CacheNeed("kv", kv_heads=self.nkv, head_dim=self.d, window=self.window)
 
+    def _part_rows(self, rt) -> int:
+        """Rows of the key slices' scratch memory, for every step the engine can have: slices x entries never exceed two CTAs
+        an SM, or the slices are 8 at most.  (One bound for decode and mixed steps: a buffer that grew would throw
+        the captured graphs away.)"""
+        return self.nq * max(2 * rt.num_sms // self.nkv + 1, 8 * rt.max_decode_rows)
+
     def _balance(self, ctx, rt, splits: int):
         """(the decode attention's ``balance``, the most slices of an entry) for a step whose entries of one token
         differ in length; (None, ``splits``) where every entry takes ``splits``."""
@@ -178,10 +184,7 @@ class GqaAttention(Part):
             # key slices (enough of them to fill the device) in one kernel, their merge in a second
             keys = min(ctx.max_kv_len, self.window) if self.window else ctx.max_kv_len
             splits = k.decode_splits(ctx.n_entries, self.nkv, rt.num_sms, self.max_splits, max_keys=keys)
-            # slices x entries never exceed two CTAs per SM, or the slices are 4 at most: that bounds
-            # the slices' scratch rows
-            # (8 slices each where their number follows the entries' lengths)
-            rows = self.nq * max(2 * rt.num_sms // self.nkv + 1, 8 * rt.max_decode_rows)
+            rows = self._part_rows(rt)
             balance, most = self._balance(ctx, rt, splits)
             part_o = rt.ws.get("attn_part_o", rows, self.d, torch.float32, cap=rows)
             part_ml = rt.ws.get("attn_part_ml", rows, 2, torch.float32, cap=rows)
@@ -221,7 +224,7 @@ class GqaAttention(Part):
             balance, most = (None, splits) if decode else self._balance(ctx, rt, splits)
             part_o = part_ml = None
             if most > 1:
-                rows = rt.max_decode_rows * self.nq * 32
+                rows = self._part_rows(rt)
                 part_o = rt.ws.get("attn_part_o", rows, self.d, torch.float32, cap=rows)
                 part_ml = rt.ws.get("attn_part_ml", rows, 2, torch.float32, cap=rows)
             k.paged_decode_attention(q, o, cache.k, cache.v, ctx.cu_q, ctx.kv_len, table,

@@ -121,11 +121,19 @@ def test_buffers_stay_where_they_are(model_folders, monkeypatch):
     run = Run(monkeypatch, model_folders("S18", "bfloat16"), max_concurrent=20)
     r, rng = run.r, np.random.default_rng(1)
     draw = lambda n: rng.integers(0, 1000, n).tolist()      # noqa: E731
-    for i, n in enumerate((250, 137, 192, 193, 40, 300, 700)):
+    for i, n in enumerate((250, 137, 192, 193, 40, 300, 700) + (30,) * 9):
         r.step([StepEntry(i, draw(n), [n - 1])])
     assert r.rt.ws.generation == 0
     r.step([StepEntry(0, draw(1), [0])])
-    assert r.rt.ws.generation == 0 and len(r._graphs) >= 1
+    kept = len(r._graphs)
+    assert kept >= 1
+    singles = [StepEntry(i, draw(1), [0]) for i in range(16)]
+    r.step(singles)                                         # 16 requests of very different lengths
+    for _ in range(2):
+        r.step([StepEntry(i, draw(1), [0]) for i in range(16)] + [StepEntry(16, draw(200), [199])])
+        r.end(16)
+    assert run.balanced["plain"] > 0
+    assert r.rt.ws.generation == 0 and len(r._graphs) > kept
     run.done()
-    for i in range(7):
+    for i in range(16):
         r.end(i)
