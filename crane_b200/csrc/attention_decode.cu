@@ -1309,6 +1309,11 @@ bool tma_path_enabled() {
     }
     return on == 1;
 }
+// Head size 128, and pages of whole tiles or tiles of whole pages (8 or 16 tokens: a piece of a tile is then a multiple of
+// the 1024 bytes the swizzle pattern repeats after).
+bool takes_tma(int d, int page_size) {
+    return d == D128 && (page_size % TILE == 0 || (page_size >= 8 && TILE % page_size == 0)) && tma_path_enabled();
+}
 // CRANE_DECODE_CLUSTER=0: the slices always go through scratch memory and the merge kernel.
 bool cluster_merge_enabled() {
     static int on = -1;
@@ -1402,10 +1407,7 @@ int launch_decode(const void* q, void* out, float* part_o, float* part_ml, const
     }
     const int cross = (!FUSED && args.cross) ? 1 : 0;
     const int nq_out = cross ? nq * nkv : nq;       // heads of the merged output
-    // pages of whole tiles, or tiles of whole pages (8 or 16 tokens: a piece of a tile is then a multiple
-    // of the 1024 bytes the swizzle pattern repeats after)
-    const bool pages_fit = page_size % TILE == 0 || (page_size >= 8 && TILE % page_size == 0);
-    const bool by_tma = D == D128 && pages_fit && tma_path_enabled();
+    const bool by_tma = takes_tma(D, page_size);
     FusedArgs fa = args;
     if (fa.tickets != nullptr && (!by_tma || cross || n_splits < 2 || n_splits > 8 || n_entries > MAX_BALANCED)) {
         fa.tickets = nullptr;                        // as many slices for every entry
@@ -1496,6 +1498,9 @@ CRANE_API int crane_paged_decode_attention_supports(int d, int nq, int nkv) {
 #undef IS
     return 0;
 }
+
+// 1 if `tickets` make a difference at this head size and page size (see crane_paged_decode_attention), else 0.
+CRANE_API int crane_paged_decode_attention_balances(int d, int page_size) { return takes_tma(d, page_size) ? 1 : 0; }
 
 // The entries with exactly one token (row cu_q[e] of q and out); entries with
 // more or no rows are skipped, so that a step's prompt portions can go to the

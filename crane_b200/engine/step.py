@@ -35,10 +35,8 @@ from ..weights.safetensors_io import DictSource
 # ``Kernels.decode_splits``).
 SHORT_CONTEXT = 2048
 SHORT_GRAPH_KEY = 1 << 20
-# A decode step whose longest context is at least half as long again as the average (and long enough to matter):
-# its attention gives long contexts more key slices, in a kernel of its own, so its graphs are others.
-UNEVEN_GRAPH_KEY = 1 << 21
-UNEVEN_KEYS = 512
+# The decode attention takes a step in one of several forms, which its graphs hold: two bits for each kind of attention.
+FORM_GRAPH_KEY = 1 << 21
 # A step whose every entry has at most this many keys in all (whole short prompts).
 SHORT_PROMPT = 64
 
@@ -89,7 +87,8 @@ class StepContext:
                                 # an attention mixer may give them to its split-KV decode kernel and
                                 # the rest to its prefill kernel
     short_prompts: bool = False     # no entry has more than 64 keys in all (whole short prompts)
-    uneven: bool = False        # the entries of one token differ in length so much that their attention is balanced
+    decode_forms: Optional[dict] = None     # by kind of attention (``form_key``), the form in which it takes the
+                                            # entries of one token (``decode_form``)
     all_single: bool = False        # every entry has exactly one token (part of a padded step's shape)
 
 
@@ -180,6 +179,9 @@ class ModelRunner:
             mixer_state = not all(getattr(mx, "decode_bucket_safe", False) for mx in keepers
                                   if any(f.kind == "state" for f in mx.cache_need().flat()))
         self._pad_with_copies = not mixer_state
+        # one attention of each kind that takes single tokens in several forms
+        self._forms_of = list({a.form_key: a for b in self.model.blocks if hasattr(b.mixer, "decode_attentions")
+                               for a in b.mixer.decode_attentions()}.values())
         self.graph_replays = 0
         self._step_done = torch.cuda.Event()       # recorded behind every step's kernels
         self._step_done.record()
@@ -321,12 +323,15 @@ class ModelRunner:
             one = cnt == 1
             if one.any() and int(m.view("kv_len", n_entries, False)[one].sum()) >= self.cfg.mixed_decode_min_keys:
                 singles = int(one.sum())
-        uneven = False
-        if not self.rt.exact:
-            held = m.view("kv_len", n_entries, False)[cnt == 1]
-            if held.size > 1 and (pad_to or singles):
-                longest = int(held.max())
-                uneven = longest >= UNEVEN_KEYS and 2 * longest * held.size > 3 * int(held.sum())
+        most_tokens = int(cnt.max())
+
+        held = m.view("kv_len", n_entries, False)[cnt == 1] if pad_to or singles else None
+
+        def decode_forms(entries: int, beside: int) -> tuple:
+            if held is None:
+                return ()
+            return tuple(a.decode_form(held, entries, beside, self.cfg.page_size, self.rt) for a in self._forms_of)
+        forms = ()
         # a small step with prompt portions: its rows are padded to 16 or a multiple of 64, its entries
         # and wanted places to a power of two, and from the second step of the same (rows,
         # entries, wanted, single-token entries) on a captured graph is replayed
@@ -345,13 +350,17 @@ class ModelRunner:
                      self._power_of_two(wanted, rows) if wanted else 0,
                      self._power_of_two(singles, self.cap_entries) if singles else 0,
                      1 if short_prompts else 0,
-                     1 if int(cnt.max()) == 1 else 0,     # nothing but single tokens: a decode step
-                     1 if uneven else 0)
+                     1 if most_tokens == 1 else 0)        # nothing but single tokens: a decode step
+            forms = decode_forms(shape[2], shape[4])
+            shape += (forms,)
             seen = self._shape_seen.get(shape, 0) + 1
             self._shape_seen[shape] = seen
             if seen >= 2:
                 key = shape
                 singles = shape[4]
+        if key is None:
+            # (single tokens alone, unpadded or in a bucket, go through the fused kernel)
+            forms = decode_forms(pad_to or n_entries, 0 if pad_to or most_tokens == 1 else singles)
         m.view("tokens", n_tokens, False)[:] = arrays[0] if len(arrays) == 1 else np.concatenate(arrays)
         # A decode step is filled up to its bucket, a small step with prompt portions to its shape, with
         # rows that belong to no entry (they write nothing into a cache) and entries without rows (no
@@ -398,20 +407,20 @@ class ModelRunner:
         ctx.graph_key = key
         ctx.single_entries = singles
         ctx.short_prompts = short_prompts
-        ctx.uneven = uneven
-        ctx.all_single = int(cnt.max()) == 1
+        ctx.decode_forms = {a.form_key: f for a, f in zip(self._forms_of, forms)}
+        ctx.all_single = most_tokens == 1
         # The host cannot launch a few hundred kernels as fast as the device runs them, busy or not, so a graph that is
         # there is always replayed (whole prompts back to back, 1.8B sizes, launched one by one / replayed, ms: 100 tokens
         # 2.65 / 2.02, 137 tokens 2.30 / 2.08, 250 tokens 2.67 / 2.21, 700 tokens 3.51 / 3.41, 2,048 tokens 7.16 / 7.11).  A
         # capture costs tens of milliseconds, so while the device is busy a shape has to come often to get one (a
         # prompt of 8,192 tokens in four portions on a new engine, 7B sizes: 110 ms, 143 with a capture in it).  Both
         # ways run the same kernels on the same rows and give the same bits.
-        ctx.replay = key is not None and (self._has_graph(key) or int(cnt.max()) == 1 or seen >= self.CAPTURE_BUSY
+        ctx.replay = key is not None and (self._has_graph(key) or most_tokens == 1 or seen >= self.CAPTURE_BUSY
                                           or self._step_done.query())
         ctx.real_want = n_want if key is None else real_want
         ctx.n_tokens, ctx.n_entries, ctx.n_want = n_tokens, n_entries, n_want
         # a padded step never counts as one of single tokens only: its filling entries have none
-        ctx.max_q_len = int(cnt.max()) if key is None else max(2, int(cnt.max()))
+        ctx.max_q_len = most_tokens if key is None else max(2, most_tokens)
         ctx.max_kv_len = int(kvl.max())
         ctx.max_positions = self.max_seq_len
         ctx.deferred_tokens = self.deferred_tokens
@@ -439,8 +448,9 @@ class ModelRunner:
                 # (a graph holds the number of key slices its attention was recorded with: short
                 # contexts, which take fewer, have graphs of their own)
                 short = ctx.max_kv_len <= SHORT_CONTEXT
-                return self._replay(ctx, ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
-                                    + (UNEVEN_GRAPH_KEY if ctx.uneven else 0))[:ctx.real_entries]
+                key = ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
+                key += sum(f * FORM_GRAPH_KEY << 2 * i for i, f in enumerate(ctx.decode_forms.values()))
+                return self._replay(ctx, key)[:ctx.real_entries]
             if ctx.graph_key is not None and ctx.replay:
                 return self._replay(ctx, ctx.graph_key)[:ctx.real_want]
             return self.model.forward(ctx, self.pools.layers)[:ctx.real_want]

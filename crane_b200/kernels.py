@@ -31,6 +31,7 @@ _SIGNATURES = {
     "crane_gemm_bf16_pair": [P, P, P, P, I, I, I, L, L, L, I, I, I, I, I, I, L, P, P],
     "crane_paged_attention_simt": [I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P, P, P],
     "crane_paged_decode_attention_supports": [I, I, I],
+    "crane_paged_decode_attention_balances": [I, I],
     "crane_paged_decode_attention": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, F, I, I, P, P, P, I, L, I, I, I, P, I, I, P, P],
     "crane_paged_prefill_attention_supports": [I, I, I],
     "crane_paged_prefill_attention": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, P, P, P, I, L, I, I, P, P, P],
@@ -1136,6 +1137,10 @@ class Kernels:
         tickets, base, slots = balance
         assert tickets.dtype == torch.int32 and tickets.numel() >= n_entries * nkv and tickets.is_contiguous()
         return [tickets.data_ptr(), int(base), int(slots)]
+
+    def decode_attention_balances(self, d: int, page_size: int) -> bool:
+        """Whether the decode attention at this head size and page size can give entries different numbers of slices."""
+        return bool(self.lib.crane_paged_decode_attention_balances(d, page_size))
 
     MOST_BALANCED = 128          # entries of a step whose slices the decode attention balances
 

@@ -14,10 +14,16 @@ from __future__ import annotations
 import math
 import os
 
+import numpy as np
 import torch
 
 from ..weights.loader import TensorSpec
 from .base import CacheNeed, Part, build_part, query_tiles, register_part
+
+
+# The least keys of the longest entry for which entries of different lengths take different numbers of slices.
+UNEVEN_KEYS = 512
+BALANCED = 1                 # a form of the decode attention (see ``GqaAttention.decode_form``)
 
 
 @register_part("mixer", "gqa_attention")
@@ -151,16 +157,47 @@ class GqaAttention(Part):
         the captured graphs away.)"""
         return self.nq * max(2 * rt.num_sms // self.nkv + 1, 8 * rt.max_decode_rows)
 
-    def _balance(self, ctx, rt, splits: int):
-        """(the decode attention's ``balance``, the most slices of an entry) for a step whose entries of one token
-        differ in length; (None, ``splits``) where every entry takes ``splits``."""
+    # ---- the form of the decode attention ---------------------------------
+    def decode_attentions(self):
+        """The attentions of this mixer that take a step's entries of one token in one of several forms (the step asks
+        each kind once and tells all, ``ctx.decode_forms``; a captured graph holds the forms it was recorded with)."""
+        return (self,)
+
+    @property
+    def form_key(self):
+        return (self.nq, self.nkv, self.d, self.window, self.max_splits)
+
+    def decode_form(self, lengths, entries: int, singles: int, page_size: int, rt) -> int:
+        """BALANCED if a step whose entries of one token hold ``lengths`` keys gives long ones more key slices, in
+        a kernel of its own: where they differ by half the average or more (behind a window: in what it leaves of
+        them) and are long enough to matter.  0: as many slices for every entry.  ``entries`` of the step, its padding
+        included; ``singles`` > 0: beside prompt portions, with about that many entries of one token."""
         k = rt.kernels
-        most = k.balanced_most(splits) if getattr(ctx, "uneven", False) and ctx.n_entries <= k.MOST_BALANCED else 0
-        if not most or self.max_splits < most:
+        held = np.minimum(lengths, self.window) if self.window else lengths
+        longest = int(held.max())
+        if longest < UNEVEN_KEYS or 2 * longest * held.size <= 3 * int(held.sum()) or entries > k.MOST_BALANCED:
+            return 0
+        splits = self._mixed_splits(rt, singles) if singles else self._fused_splits(rt, entries, int(lengths.max()))
+        most = k.balanced_most(splits)
+        return BALANCED if 0 < most <= self.max_splits and k.decode_attention_balances(self.d, page_size) else 0
+
+    def _fused_splits(self, rt, entries: int, max_kv_len: int) -> int:
+        keys = min(max_kv_len, self.window) if self.window else max_kv_len
+        return rt.kernels.decode_splits(entries, self.nkv, rt.num_sms, self.max_splits, max_keys=keys)
+
+    def _mixed_splits(self, rt, singles: int) -> int:
+        # at most 8 slices: at head size 128 they merge inside a cluster without scratch
+        return min(8, rt.kernels.decode_splits(singles, self.nkv, rt.num_sms, self.max_splits))
+
+    def _balance(self, ctx, rt, splits: int):
+        """(the decode attention's ``balance``, the most slices of an entry); (None, ``splits``) where every entry takes
+        ``splits``."""
+        k = rt.kernels
+        if (getattr(ctx, "decode_forms", None) or {}).get(self.form_key) != BALANCED:
             return None, splits
         # (kept by the workspace: zeros, which every launch leaves as zeros)
         tickets = rt.ws.zeros("attn_tickets", k.MOST_BALANCED, self.nkv, torch.int32)
-        return (tickets, splits, 2 * rt.num_sms), most
+        return (tickets, splits, 2 * rt.num_sms), k.balanced_most(splits)
 
     def forward(self, h, ctx, cache, rt, hold: bool = False):
         n = h.shape[0]
@@ -182,8 +219,7 @@ class GqaAttention(Part):
         if decode and self.d % 4 == 0:
             # single decoded tokens: rotary encoding, head norms, the cache write, attention over
             # key slices (enough of them to fill the device) in one kernel, their merge in a second
-            keys = min(ctx.max_kv_len, self.window) if self.window else ctx.max_kv_len
-            splits = k.decode_splits(ctx.n_entries, self.nkv, rt.num_sms, self.max_splits, max_keys=keys)
+            splits = self._fused_splits(rt, ctx.n_entries, ctx.max_kv_len)
             rows = self._part_rows(rt)
             balance, most = self._balance(ctx, rt, splits)
             part_o = rt.ws.get("attn_part_o", rows, self.d, torch.float32, cap=rows)
@@ -219,8 +255,7 @@ class GqaAttention(Part):
             if decode:
                 splits = max(1, min(32, (2 * rt.num_sms) // max(1, ctx.n_entries * self.nkv)))
             else:
-                # at most 8 slices: at head size 128 they merge inside a cluster without scratch
-                splits = min(8, k.decode_splits(singles, self.nkv, rt.num_sms, self.max_splits))
+                splits = self._mixed_splits(rt, singles)
             balance, most = (None, splits) if decode else self._balance(ctx, rt, splits)
             part_o = part_ml = None
             if most > 1:

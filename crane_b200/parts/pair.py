@@ -41,6 +41,9 @@ class ParallelPair(Part):
         keeps = [m for m in (self.left, self.right) if any(f.kind == "state" for f in m.cache_need().flat())]
         return all(getattr(m, "decode_bucket_safe", False) for m in keeps)
 
+    def decode_attentions(self):
+        return tuple(a for m in (self.left, self.right) if hasattr(m, "decode_attentions") for a in m.decode_attentions())
+
     def load(self, weights, rt):
         a, p = self.params, self.prefix
         self.left.load(weights, rt)

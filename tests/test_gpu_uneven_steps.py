@@ -137,3 +137,69 @@ def test_buffers_stay_where_they_are(model_folders, monkeypatch):
     run.done()
     for i in range(16):
         r.end(i)
+
+
+def decode_graphs(r):
+    return [k for k in r._graphs if isinstance(k, int)]
+
+
+@pytest.mark.parametrize("change,n", [(dict(num_key_value_heads=4), 3), (dict(head_dim=64), 9)])
+def test_no_second_graph_of_the_same_kernels(change, n, tmp_path, monkeypatch):
+    """Three requests at four key/value heads take 8 key slices each however long they are, and at head size 64 nothing is
+    balanced: steps of even and of uneven lengths replay one graph."""
+    from crane_b200.engine import StepEntry
+    from crane_b200.weights.random_init import write_model_folder
+    folder = write_model_folder(str(tmp_path / "m"), dict(CFG, **change), 3, "bfloat16", std=0.05, norm_std=0.05)
+    run = Run(monkeypatch, folder)
+    r = run.r
+    for i in range(2 * n):
+        r.step([StepEntry(i, [(7 * j + i) % 300 for j in range(700 if i == 0 else 20 + i)], [])])
+    before = r.graph_replays
+    for _ in range(3):
+        for first in (0, n):                                # n requests with the long one, then n without
+            r.step([StepEntry(i, [5], [0]) for i in range(first, first + n)])
+    assert run.balanced == {"fused": 0, "plain": 0}
+    assert len(decode_graphs(r)) == 1 and r.graph_replays == before + 5
+    run.done()
+    for i in range(2 * n):
+        r.end(i)
+
+
+def test_balanced_and_windowed_attention_in_one_step(monkeypatch):
+    """Layers that alternate between all earlier positions and a window of 100: lengths of 5 to 900 are balanced in the former
+    and equal enough in the latter; decode and mixed steps against the plain computation."""
+    import test_gpu_window_layers as tw
+    from crane_b200.config import EngineConfig, resolve
+    from crane_b200.engine import ModelRunner, StepEntry
+    from crane_b200.parts import model_manifest
+    from crane_b200.weights.random_init import random_tensors
+    cfg = dict(tw.CFG, hidden=128, heads=16, kv_heads=8, head_dim=128, window=100, max_pos=1024, layers=2)
+    monkeypatch.setattr(tw, "CFG", cfg)
+    tw.register()
+    tensors = random_tensors(model_manifest(resolve(cfg).build_spec(cfg)), 9, torch.bfloat16, std=0.08, norm_std=0.05)
+    w = {k: v.double().numpy() for k, v in tensors.items()}
+    r = ModelRunner(None, EngineConfig(dtype="bfloat16", page_size=32, num_pages=200, max_concurrent=20,
+                                       max_batched_tokens=1024), config=cfg, tensors=tensors)
+    rng = np.random.default_rng(2)
+    lens = SHORT + LONG
+    seqs = [rng.integers(0, 120, n + 10).tolist() for n in lens]
+    want = [tw.plain_logits(w, s) for s in seqs]
+    forms = []
+    prepare = r.prepare
+    monkeypatch.setattr(r, "prepare", lambda *a, **kw: forms.append(prepare(*a, **kw)) or forms[-1])
+
+    def check(got, places):
+        for g, (i, p) in zip(got.float().cpu().numpy(), places):
+            assert np.abs(g - want[i][p]).max() / np.abs(want[i]).max() < 3e-2, (i, p)
+    for i, n in enumerate(lens):
+        check(r.step([StepEntry(i, seqs[i][:n], [n - 1])]), [(i, n - 1)])
+    for t in range(6):
+        entries = [StepEntry(i, [seqs[i][n + t]], [0]) for i, n in enumerate(lens)]
+        if t >= 3:
+            entries.append(StepEntry(50 + t, seqs[10][:40], []))
+        check(r.step(entries), [(i, n + t) for i, n in enumerate(lens)])
+        assert {k[3]: f for k, f in forms[-1].decode_forms.items()} == {0: 1, 100: 0}
+    r.rt.check_errors()
+    for i in list(range(len(lens))) + [53, 54, 55]:
+        r.end(i)
+    r.table.check()

@@ -110,3 +110,49 @@ def test_few_rows_plan_and_its_bound():
     # one size, three numbers of slices: what a buffer made for the first caller would not hold
     assert [Kernels.few_rows_plan(m, 2048, 2048, SMS) for m in (1, 137, 250)] == [(16, 8), (64, 6), (64, 4)]
     assert Kernels.few_rows_plan(250, 4096, 14336, SMS) == (256, 8)        # a long share of the inner dimension: one tile of tokens
+
+
+def _attention(nkv=8, window=0, d=128, max_splits=64):
+    from crane_b200.parts.attention import GqaAttention
+    a = GqaAttention.__new__(GqaAttention)
+    a.nq, a.nkv, a.d, a.window, a.max_splits = 2 * nkv, nkv, d, window, max_splits
+    return a
+
+
+class _K(Kernels):
+    def __init__(self):
+        pass
+
+    def decode_attention_balances(self, d, page_size):
+        return d == 128 and (page_size % 32 == 0 or page_size in (8, 16))
+
+
+class _Rt:
+    num_sms, kernels = SMS, _K()
+
+
+def test_decode_form():
+    """A step's decode attention is a kernel (and a graph) of its own only where the slices really differ."""
+    form = lambda a, lens, entries, singles=0, page=64: a.decode_form(np.array(lens), entries, singles, page, _Rt)    # noqa: E731
+    uneven, even = [2000] + [100] * 12, [900] * 13
+    assert form(_attention(), uneven, 16) == 1 and form(_attention(), even, 16) == 0
+    assert form(_attention(), uneven, 16, singles=16) == 1                  # beside prompt portions
+    assert form(_attention(), [511] + [20] * 12, 16) == 0                   # too short to matter
+    assert form(_attention(), [600] * 5 + [401] * 5, 10) == 0               # 1.2 times the average
+    assert form(_attention(nkv=4), [2000, 100, 100], 4) == 0                # few entries: 8 slices each, merged in a cluster
+    assert form(_attention(nkv=4), [2000] + [100] * 31, 32) == 1
+    assert form(_attention(), [2000] + [100] * 128, 132) == 0               # more entries than the kernel balances
+    assert form(_attention(d=64), uneven, 16) == 0 and form(_attention(), uneven, 16, page=4) == 0
+    assert form(_attention(max_splits=3), uneven, 16) == 0
+    # behind a window entries beyond it are equal
+    assert form(_attention(window=100), uneven, 16) == 0
+    assert form(_attention(window=600), [2000] * 6 + [700] * 7, 16) == 0
+    assert form(_attention(window=1500), [1500] + [100] * 12, 16) == 1
+    # the slices it says yes to are what the forward pass takes: never more than the scratch memory is made for
+    for nkv in (1, 2, 4, 8):
+        for n in range(2, 129):
+            a = _attention(nkv=nkv)
+            for singles in (0, n):
+                splits = a._mixed_splits(_Rt, singles) if singles else a._fused_splits(_Rt, n, 5000)
+                if form(a, [4000] + [10] * (n - 1), n, singles):
+                    assert splits < Kernels.balanced_most(splits) <= 8
