@@ -160,7 +160,7 @@ class ModelRunner:
         self.steps = 0
         # decode steps (one token per entry) of the bfloat16 path replay a captured graph
         self._graphs: Dict[object, tuple] = {}
-        self._shape_seen: Dict[tuple, int] = {}      # how often a shape of small step has come
+        self._shape_seen: Dict[object, int] = {}     # how often a shape of small step has come, or a decode step's form
         self._graph_generation = -1
         has_state = any(f.kind == "state" for n in self.model.cache_needs() for f in n.flat())
         self._graphs_ok = (self.cfg.use_cuda_graphs and not self.rt.exact and self.model.capturable()
@@ -449,8 +449,8 @@ class ModelRunner:
                 # contexts, which take fewer, have graphs of their own)
                 short = ctx.max_kv_len <= SHORT_CONTEXT
                 key = ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
-                key += sum(f * FORM_GRAPH_KEY << 2 * i for i, f in enumerate(ctx.decode_forms.values()))
-                return self._replay(ctx, key)[:ctx.real_entries]
+                form = sum(f * FORM_GRAPH_KEY << 2 * i for i, f in enumerate(ctx.decode_forms.values()))
+                return self._replay(ctx, self._form_graph(key, form))[:ctx.real_entries]
             if ctx.graph_key is not None and ctx.replay:
                 return self._replay(ctx, ctx.graph_key)[:ctx.real_want]
             return self.model.forward(ctx, self.pools.layers)[:ctx.real_want]
@@ -478,6 +478,20 @@ class ModelRunner:
 
     def _has_graph(self, key) -> bool:
         return key in self._graphs and self._graph_generation == self.rt.ws.generation
+
+    def _form_graph(self, key: int, form: int) -> int:
+        """The graph for a decode step whose attention takes the form ``form``: its own, or, until this form has come
+        CAPTURE_BUSY times, one of the same bucket in another form if there is one.  (Every form serves every step; they
+        differ in how fast.  Lengths that drift across a rule's line would else stop all requests for a capture.)"""
+        own = key + form
+        if self._has_graph(own):
+            return own
+        others = [k for k in self._graphs if isinstance(k, int) and k % FORM_GRAPH_KEY == key and self._has_graph(k)]
+        if others:
+            seen = self._shape_seen[own] = self._shape_seen.get(own, 0) + 1
+            if seen < self.CAPTURE_BUSY:
+                return others[-1]
+        return own
 
     MAX_SHAPE_GRAPHS = 256      # graphs of small steps kept; the least recently used one goes first
 

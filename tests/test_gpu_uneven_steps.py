@@ -203,3 +203,59 @@ def test_balanced_and_windowed_attention_in_one_step(monkeypatch):
     for i in list(range(len(lens))) + [53, 54, 55]:
         r.end(i)
     r.table.check()
+
+
+def test_a_batch_that_crosses_the_line_keeps_its_graph_at_first(uneven_model, monkeypatch):
+    """Steps of ten requests that turn uneven replay the graph their bucket has; the balanced one is captured when they have
+    come often.  The same the other way round, in a bucket that has the balanced graph alone."""
+    run = Run(monkeypatch, *uneven_model)
+    r, short, long_ = run.r, list(range(10)), [10, 11, 12]
+    run.prefill(short + long_, SHORT + LONG)
+    even, uneven = {i: 1 for i in short[:9]}, {i: 1 for i in short[:6] + long_}
+    captures = r.graph_captures
+    run.step(even)
+    assert r.graph_captures == captures + 1
+    for t in range(1, r.CAPTURE_BUSY):
+        run.step(uneven)
+        assert r.graph_captures == captures + 1 and run.balanced["fused"] == 0
+    run.step(uneven)
+    assert r.graph_captures == captures + 2 and run.balanced["fused"] > 0
+    replays = r.graph_replays
+    for _ in range(3):
+        run.step(uneven)
+        run.step(even)
+    assert (r.graph_captures, r.graph_replays) == (captures + 2, replays + 6) and len(decode_graphs(r)) == 2
+    for k in decode_graphs(r):                              # (as in an engine that has met uneven steps only)
+        if k < 1 << 21:
+            del r._graphs[k]
+    for _ in range(3):
+        run.step(even)
+    assert r.graph_captures == captures + 2
+    run.done()
+
+
+def test_replay_while_the_device_is_busy(uneven_model, monkeypatch):
+    """Short prompts one after the other without a look at their results: a shape is captured on a busy device when it has
+    come 16 times, not before, and then replayed; up to 16 tokens are padded to 16 rows.  The logits are the plain ones."""
+    class Busy:
+        def query(self):
+            return False
+
+        def record(self):
+            pass
+    run = Run(monkeypatch, *uneven_model)
+    r = run.r
+    monkeypatch.setattr(r, "_step_done", Busy())
+    kept = []
+    for t in range(30):
+        i, n = t % len(run.seqs), 1 + (7 * t) % 16
+        if n == 1:
+            n = 16                                          # (single tokens are decode steps)
+        kept.append((run.step({i: n}, check=False).clone(), [(i, n - 1)]))
+        r.end(i)
+        run.at[i] = 0
+        assert r.graph_captures == (1 if t >= 15 else 0)
+    assert r.graph_replays == 14 and [k[:2] for k in r._graphs] == [("rows", 16)]
+    for got, places in kept:
+        run.compare(got, places)
+    run.done()
