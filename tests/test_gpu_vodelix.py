@@ -490,3 +490,33 @@ def test_command_line(model_folders):
     p = subprocess.run(cmd, capture_output=True, text=True, timeout=300)
     assert p.returncode == 0, p.stderr[-3000:]
     assert p.stdout.strip().splitlines()[-1] == ",".join(map(str, pv.greedy_generate(cfg, w, [5, 6, 7], 6)[3:]))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hidden,parts", [(2048, 3), (2048, 0), (1028, 4), (3072, 5), (1030, 2), (4104, 1)])
+def test_add_normed_norm_many_rows(K, dtype, hidden, parts):
+    """More rows than a step of few tokens: rows wider than a block's threads times four, with partial sums read 16 bytes at a
+    time where rows are whole 16-byte pieces and one by one where they are not."""
+    from crane_b200.kernels import Partials
+    rng = np.random.default_rng(hidden + parts)
+    n = 70
+    x = rng.standard_normal((n, hidden)).astype(np.float32) * 3
+    wd, wo = (1 + 0.3 * rng.standard_normal(hidden).astype(np.float32) for _ in range(2))
+    p = _dev(rng.standard_normal((max(parts, 1), n, hidden)))
+    if parts:
+        total = p[0].clone()
+        for i in range(1, parts):
+            total = total + p[i]                                             # in slice order, rounded once
+        delta, dn = Partials(p), total.to(dtype).double().cpu().numpy()
+    else:
+        delta = p[0].to(dtype)
+        dn = delta.double().cpu().numpy()
+    new = x + pv.rms_norm(dn, wd, 1e-6)
+    xd, out = _dev(x), torch.empty(n, hidden, dtype=dtype, device=DEV)
+    raw = torch.empty_like(out)
+    K.add_normed_norm(xd, delta, _dev(wd), 1e-6, _dev(wo), 1e-5, out, raw)
+    # (bounds as in the test above)
+    tol = 2e-5 if dtype == torch.float32 else 2e-2
+    assert np.abs(xd.cpu().numpy() - new).max() < 1e-5 * np.abs(new).max()
+    assert np.abs(out.double().cpu().numpy() - pv.rms_norm(new, wo, 1e-5)).max() < tol * 4
+    assert np.abs(raw.double().cpu().numpy() - new).max() < tol * np.abs(new).max()
