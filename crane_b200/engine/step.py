@@ -26,6 +26,7 @@ from ..cache.pools import CachePools, bytes_per_page, group_layers
 from ..config import EngineConfig, read_config_json, resolve
 from ..config.engine_config import parse_memory_limit
 from ..parts import DecoderModel, Runtime
+from ..parts.attention import UNEVEN_KEYS
 from ..weights.loader import open_folder
 from ..weights.safetensors_io import DictSource
 
@@ -88,7 +89,7 @@ class StepContext:
                                 # the rest to its prefill kernel
     short_prompts: bool = False     # no entry has more than 64 keys in all (whole short prompts)
     decode_forms: Optional[dict] = None     # by kind of attention (``form_key``), the form in which it takes the
-                                            # entries of one token (``decode_form``)
+                                            # entries of one token (``decode_form``); None: 0 for all
     all_single: bool = False        # every entry has exactly one token (part of a padded step's shape)
 
 
@@ -317,7 +318,8 @@ class ModelRunner:
         # attention, in tiles of 64 rows and several CTAs per SM, beats the tcgen05 kernel's 128-row
         # tiles there (see the attention part); it is part of a small step's shape, since a graph holds
         # the kernel it was recorded with.
-        short_prompts = int(m.view("kv_len", n_entries, False).max()) <= SHORT_PROMPT
+        most_keys = int(m.view("kv_len", n_entries, False).max())
+        short_prompts = most_keys <= SHORT_PROMPT
         singles = 0
         if not pad_to and not self.rt.exact:
             one = cnt == 1
@@ -325,12 +327,15 @@ class ModelRunner:
                 singles = int(one.sum())
         most_tokens = int(cnt.max())
 
-        held = m.view("kv_len", n_entries, False)[cnt == 1] if pad_to or singles else None
+        held = None
+        if (pad_to or singles > 1) and real_entries > 1 and most_keys >= UNEVEN_KEYS:
+            held = m.view("kv_len", n_entries, False)[cnt == 1]
 
         def decode_forms(entries: int, beside: int) -> tuple:
             if held is None:
                 return ()
-            return tuple(a.decode_form(held, entries, beside, self.cfg.page_size, self.rt) for a in self._forms_of)
+            forms = tuple(a.decode_form(held, entries, beside, self.cfg.page_size, self.rt) for a in self._forms_of)
+            return forms if any(forms) else ()
         forms = ()
         # a small step with prompt portions: its rows are padded to 16 or a multiple of 64, its entries
         # and wanted places to a power of two, and from the second step of the same (rows,
@@ -407,7 +412,7 @@ class ModelRunner:
         ctx.graph_key = key
         ctx.single_entries = singles
         ctx.short_prompts = short_prompts
-        ctx.decode_forms = {a.form_key: f for a, f in zip(self._forms_of, forms)}
+        ctx.decode_forms = {a.form_key: f for a, f in zip(self._forms_of, forms)} if forms else None
         ctx.all_single = most_tokens == 1
         # The host cannot launch a few hundred kernels as fast as the device runs them, busy or not, so a graph that is
         # there is always replayed (whole prompts back to back, 1.8B sizes, launched one by one / replayed, ms: 100 tokens
@@ -449,7 +454,9 @@ class ModelRunner:
                 # contexts, which take fewer, have graphs of their own)
                 short = ctx.max_kv_len <= SHORT_CONTEXT
                 key = ctx.graph_bucket + (SHORT_GRAPH_KEY if short else 0)
-                form = sum(f * FORM_GRAPH_KEY << 2 * i for i, f in enumerate(ctx.decode_forms.values()))
+                form = 0
+                if ctx.decode_forms:
+                    form = sum(f * FORM_GRAPH_KEY << 2 * i for i, f in enumerate(ctx.decode_forms.values()))
                 return self._replay(ctx, self._form_graph(key, form))[:ctx.real_entries]
             if ctx.graph_key is not None and ctx.replay:
                 return self._replay(ctx, ctx.graph_key)[:ctx.real_want]
