@@ -206,9 +206,9 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 }
 
 // Slices of the inner dimension: the number for which the rounds over the SMs take the least time, a CTA an SM
-// (fewer slices where more gain little); a slice has at least 8 blocks.  Of N and K alone, so that M does not
-// change a sum.  A cluster lies in one GPC (at least 16 SMs on this device), so clusters of 3, 5, 6 and 7 leave SMs
-// idle.  (97 tokens, 12288 x 2048: 3 slices are 288 CTAs, but only 135 of them run at once; the SMs were busy for
+// (fewer slices where more gain little); a slice has at least 8 blocks.  Of N and K alone, so that neither M nor
+// the device at hand changes a sum: 148 SMs and their GPCs are those of the device the times were taken on.  A cluster
+// lies in one GPC (at least 16 SMs there), so clusters of 3, 5, 6 and 7 leave SMs idle.  (97 tokens, 12288 x 2048: 3 slices are 288 CTAs, but only 135 of them run at once; the SMs were busy for
 // 64 % of the kernel's 245 us.)
 int f32_slices(int N, int K) {
     const int tiles = (N + FN - 1) / FN, blocks = (K + FK - 1) / FK;

@@ -968,6 +968,16 @@ int launch_pair(const void* A, const void* B, int rows_a, int rows_b, int k, lon
     return crane_launch_cluster(kern, dim3(2 * pairs), dim3(NUM_THREADS), smem, dim3(2, 1, 1), st, ma, mb, p);
 }
 
+int sm_count() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    return sms;
+}
+
 template <bool OUT_F32, bool TRANSPOSED>
 int dispatch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, dim3 grid,
                 cudaStream_t st) {
@@ -979,9 +989,11 @@ int dispatch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, const Gemm
         case 64: return launch<64, 4, OUT_F32, TRANSPOSED>(ma, mb, p, grid, st);
         // more tiles than SMs: three stages, so that two CTAs share an SM and one's first operands and epilogue overlap
         // the other's products (whole prompt of 700 tokens, 2048 x 6144 in 3 slices, 288 tiles: 0.06 ms faster than tiles of 256
-        // tokens on half as many SMs; with six stages, one CTA at a time, 0.32 ms slower)
+        // tokens on half as many SMs; with six stages, one CTA at a time, 0.32 ms slower; a decode step's products at 65 /
+        // 128 tokens, three stages against six, us: 12288 x 3072 in 3 slices 19.4 / 21.8 against 25.8 / 29.8, 4096 x 14336
+        // 27.6 / 30.7 against 34.0 / 38.5, a head of 128167 x 4096 186 / 201 against 201 / 222)
         case 128:
-            if (grid.x * grid.y * grid.z > 148u) return launch<128, 3, OUT_F32, TRANSPOSED>(ma, mb, p, grid, st);
+            if ((int)(grid.x * grid.y * grid.z) > sm_count()) return launch<128, 3, OUT_F32, TRANSPOSED>(ma, mb, p, grid, st);
             return launch<128, 6, OUT_F32, TRANSPOSED>(ma, mb, p, grid, st);
         case 256: return launch<256, 4, OUT_F32, TRANSPOSED>(ma, mb, p, grid, st);
     }
@@ -1077,9 +1089,9 @@ CRANE_API int crane_gemm_bf16_tcgen05(const void* A, const void* B, const float*
                       : dispatch_bn<false, false>(bn, ma, mb, p, grid, st);
 }
 
-// The same product as crane_gemm_bf16_tcgen05 for many tokens (bf16 output, untransposed, no
-// slices) on pairs of SMs: 256 x bn tiles, bn in 128, 192, 224, 256, or (tile_rows 512) 512 x bn
-// tiles, bn in 192, 224, 256.  epilogue as there.
+// The same product as crane_gemm_bf16_tcgen05 for many tokens (untransposed) on pairs of SMs: 256 x bn tiles, bn in
+// 128, 192, 224, 256, or (tile_rows 512) 512 x bn tiles, bn in 192, 224, 256.  bf16 output; epilogue as there.
+// slices > 1: float partial sums [slices][rows_a][ld_out], split_stride apart (256 x 256 tiles, no bias, epilogue or groups).
 CRANE_API int crane_gemm_bf16_pair(const void* A, const void* B, const float* bias, void* out, int rows_a,
                                    int rows_b, int k, long long lda, long long ldb, long long ld_out,
                                    int bn, int tile_rows, int epilogue, int group_features, int group_rows,

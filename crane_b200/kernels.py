@@ -923,7 +923,7 @@ class Kernels:
                      bn: int = 128, silu_mul: bool = False, prefetch=None, tile_rows: int = 128,
                      group_features: int = 0, group_rows: int = 0) -> None:
         """out[M,N] = x[M,K] @ w[N,K]^T (+ bias).  ``swap``: the weight fills the
-        128-row side of the MMA and ``bn`` (16..64) covers the tokens.  With
+        128-row side of the MMA and ``bn`` (16..256) covers the tokens.  With
         ``split_k`` > 1 ``out`` is float [slices, M, N] of partial sums.
         ``silu_mul``: w's rows come as 16 gate rows then the 16 up rows of the same
         features, and out[M, N/2] = silu(gate) * up.  ``prefetch``: (address,

@@ -283,13 +283,13 @@ def test_overlapped_steps_on_a_lagging_device_change_no_token(dtype, model_folde
 @pytest.mark.parametrize("name", ["B", "C", "S18", "D144"])
 def test_small_steps_replay_graphs_with_the_same_logits(name, model_folders):
     """Steps with prompt portions of up to graph_max_tokens tokens are padded to
-    a multiple of 64 rows and, from the second step of a shape on, replay a
+    16 rows or a multiple of 64 and, from the second step of a shape on, replay a
     captured graph: prompts of different lengths under one shape, then a
     portion beside decoded tokens, then decoding, give the logits of an engine
     that launches every step kernel by kernel; the padding rows write nothing
     into the cache (the decoded tokens that follow read it).  Every step here
-    finds the device idle (its results are read each time): only then does a
-    step take a graph."""
+    finds the device idle (its results are read each time), so a shape is
+    captured at its second coming; a busy device: test_gpu_uneven_steps.py."""
     from crane_b200.engine import StepEntry
     folder = model_folders(name, "bfloat16")
     rng = np.random.default_rng(3)
@@ -306,7 +306,7 @@ def test_small_steps_replay_graphs_with_the_same_logits(name, model_folders):
         for i in (20, 21, 22):                                  # portions of which nothing is wanted
             p = rng.integers(0, vocab, 150).tolist()
             assert r.step([StepEntry(i, p[:100], [])]).shape[0] == 0
-            torch.cuda.synchronize()                            # a graph is taken only while the device idles
+            torch.cuda.synchronize()                            # (idle: captured at once)
             out.append(r.step([StepEntry(i, p[100:], [49])]).float().cpu())
             r.end(i)
         for t, n_single in enumerate((4, 3, 2, 4)):             # single tokens beside a portion of 30:

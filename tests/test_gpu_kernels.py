@@ -1224,3 +1224,43 @@ def test_gemm_pair_behind_kernels_that_end_raggedly(K, err):
         torch.cuda.synchronize()
         assert torch.equal(parts, first)
     assert int(err.item()) == 0
+
+
+# products with the weights on the 128-row side: tiles of 128 tokens in three stages, two CTAs an SM (more than 148 CTAs), with a last
+# tile of tokens that is not full and features past the last tile; the same in six stages (fewer CTAs); several tiles of 64 tokens
+@pytest.mark.parametrize("bn,M,N,K_,slices", [(128, 700, 2048, 6144, 3), (128, 300, 2040, 2048, 4), (128, 65, 4096, 1032, 5),
+                                              (128, 300, 1000, 640, 3), (64, 137, 2048, 2048, 6), (64, 250, 2056, 1032, 4),
+                                              (64, 192, 12288, 264, 1)])
+def test_gemm_tcgen05_swapped_many_tiles_of_tokens(K, err, bn, M, N, K_, slices):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(M + N)
+    a, w = (torch.randn(r, K_, generator=g, device=DEV).bfloat16() for r in (M, N))
+    bias = torch.randn(N, generator=g, device=DEV)
+    want = a.double() @ w.double().T + bias.double()
+    if slices == 1:
+        out = torch.full((M + 1, N), 7.0, device=DEV, dtype=torch.bfloat16)
+        K.gemm_tcgen05(a, w, bias, out[:M], err, swap=True, bn=bn)
+        assert rel_err(out[:M], want) < 5e-3 and bool((out[M] == 7.0).all())
+    else:
+        parts = torch.full((slices + 1, M, N), 7.0, device=DEV)
+        K.gemm_tcgen05(a, w, bias, parts[:slices], err, split_k=slices, swap=True, bn=bn)
+        assert rel_err(parts[:slices].sum(0), want) < acc_tol(K_) and bool((parts[slices] == 7.0).all())
+        blocks = (K_ + 63) // 64
+        for s in range(slices):                              # (each slice its own blocks of the inner dimension)
+            lo, hi = s * blocks // slices * 64, min(K_, (s + 1) * blocks // slices * 64)
+            part = a[:, lo:hi].double() @ w[:, lo:hi].double().T + (bias.double() if s == 0 else 0.0)
+            assert rel_err(parts[s], part) < acc_tol(hi - lo)
+    assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("M", [137, 250])
+def test_gemm_tcgen05_grouped_tiles_of_64_tokens(K, err, M):
+    """Groups of features that read rows of their own, several tiles of 64 tokens, in slices."""
+    N, K_, features, slices = 1024, 520, 256, 3
+    xs = torch.randn(4, M, K_, device=DEV).bfloat16()
+    w = torch.randn(N, K_, device=DEV).bfloat16()
+    parts = torch.full((slices, M, N), 7.0, device=DEV)
+    K.gemm_tcgen05(xs[0], w, None, parts, err, split_k=slices, swap=True, bn=64, group_features=features, group_rows=M)
+    want = torch.cat([xs[g].double() @ w[g * features:(g + 1) * features].double().T for g in range(4)], dim=1)
+    assert int(err.item()) == 0
+    assert rel_err(parts.sum(0), want) < acc_tol(K_)

@@ -220,7 +220,7 @@ def test_a_mixer_with_state_replays_graphs_when_it_bears_padding():
         out.append(r.step([StepEntry(3, reqs[3][:12], [11]), StepEntry(1, reqs[1][20:30], [9])]).float().cpu())
         pos = {1: 30, 2: 9, 3: 12}
         for live in ([1, 2, 3], [1, 2, 3], [1, 2, 3], [1, 3], [1, 3], [1, 3], [2], [1, 2, 3], [1, 2, 3]):
-            torch.cuda.synchronize()                      # an idle device: a step of a seen shape replays its graph
+            torch.cuda.synchronize()                      # (idle: a shape that has been seen is captured)
             out.append(r.step([StepEntry(i, [reqs[i][pos[i]]], [0]) for i in live]).float().cpu())
             for i in live:
                 pos[i] += 1
