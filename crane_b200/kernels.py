@@ -7,6 +7,7 @@ raises.
 """
 from __future__ import annotations
 
+import functools
 import os
 from dataclasses import dataclass
 from ctypes import c_float, c_int, c_longlong, c_void_p
@@ -784,11 +785,13 @@ class Kernels:
     def few_rows_tile(m: int) -> int:
         return 16 if m <= 16 else 32 if m <= 32 else 64 if m <= 64 else 128 if m <= 128 else 256
 
-    @classmethod
-    def few_rows_plan(cls, m: int, n: int, k: int, sms: int):
+    # (both kept for the sizes that have come: the search for slices takes longer than launching the product)
+    @staticmethod
+    @functools.lru_cache(maxsize=8192)
+    def few_rows_plan(m: int, n: int, k: int, sms: int):
         """(tokens of a tile, slices of the inner dimension) of a product of at most 256 tokens, whose weight rows fill the
         MMA's 128-wide side and whose inner dimension is cut until every SM has a tile to stream."""
-        bn, tiles, row_tiles = cls.few_rows_tile(m), -(-n // 128), -(-m // 64)
+        bn, tiles, row_tiles = Kernels.few_rows_tile(m), -(-n // 128), -(-m // 64)
         most = 2 * sms // (tiles * row_tiles)
         if bn == 256 and most >= 1 and (most >= 3 or k // most <= 4096):
             # More than 128 tokens: tiles of 64, two CTAs an SM, fewer slices of the inner dimension, instead of
@@ -799,12 +802,13 @@ class Kernels:
             # 5.01 -> 5.16, hence the second condition.
             return 64, min(8, most, max(1, k // 256))
         # at most 8: the consumers of partial sums fetch eight slices at a time
-        return bn, min(cls.slices_for(tiles, k, sms), 8)
+        return bn, min(Kernels.slices_for(tiles, k, sms), 8)
 
-    @classmethod
-    def few_rows_most_slices(cls, n: int, k: int, sms: int) -> int:
+    @staticmethod
+    @functools.lru_cache(maxsize=1024)
+    def few_rows_most_slices(n: int, k: int, sms: int) -> int:
         """The most slices that ``few_rows_plan`` gives any number of tokens (it changes with the kind of tile alone)."""
-        return max(cls.few_rows_plan(m, n, k, sms)[1] for m in (1, 129, 193))
+        return max(Kernels.few_rows_plan(m, n, k, sms)[1] for m in (1, 129, 193))
 
     PAIR_TILES = (256, 224, 192, 128)
 
