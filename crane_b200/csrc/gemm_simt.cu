@@ -72,9 +72,10 @@ gemm_nt_kernel(const TA* __restrict__ A, const TA* __restrict__ W, const float* 
 }
 
 // ---- float operands, rows of whole 16-byte pieces --------------------------------------------------
-// What bounds it: with few rows the weights' way from DRAM; with many the operands' way from shared memory
-// into registers (16 bytes a lane take four clocks of an SM, whether or not the lanes read the same ones), and
-// behind it the FP32 cores.  Whole prompts at hidden 2048, inner 6144, 32 layers, 32-bit: 97 tokens 39.3 -> 22.2 ms
+// What bounds it: with few rows the weights' way from DRAM; with many the latency of the operands' way from shared memory
+// into registers (16 bytes a lane take four clocks of an SM, whether or not the lanes read the same ones) and of a barrier
+// every 32 k, which two warps a scheduler do not cover: 97 x 12288 x 2048 takes 187 us with the multiply-add pipe 48 %, issue
+// slots 42 % and shared memory 40 % of the SMs' active cycles.  Whole prompts at hidden 2048, inner 6144, 32 layers, 32-bit: 97 tokens 39.3 -> 22.2 ms
 // (17.0 with the slices below and wider loads in the attention), 24 tokens 34.5 -> 6.1 ms; `gemm_nt_kernel`, which
 // reads every operand 4 bytes at a time and has no slices, took nearly all of it before.
 //
@@ -208,8 +209,8 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 // Slices of the inner dimension: the number for which the rounds over the SMs take the least time, a CTA an SM
 // (fewer slices where more gain little); a slice has at least 8 blocks.  Of N and K alone, so that neither M nor
 // the device at hand changes a sum: 148 SMs and their GPCs are those of the device the times were taken on.  A cluster
-// lies in one GPC (at least 16 SMs there), so clusters of 3, 5, 6 and 7 leave SMs idle.  (97 tokens, 12288 x 2048: 3 slices are 288 CTAs, but only 135 of them run at once; the SMs were busy for
-// 64 % of the kernel's 245 us.)
+// lies in one GPC (at least 16 SMs there), so clusters of 3, 5, 6 and 7 leave SMs idle.  (97 tokens, 12288 x 2048: 3 slices are 288
+// CTAs, but only 135 of them run at once; the SMs were busy for 64 % of the kernel's 245 us.)
 int f32_slices(int N, int K) {
     const int tiles = (N + FN - 1) / FN, blocks = (K + FK - 1) / FK;
     int best = 1;
