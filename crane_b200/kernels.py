@@ -27,7 +27,9 @@ _SIGNATURES = {
     "crane_silu_mul": [I, P, P, I, L, P, I, I, I, P],
     "crane_to_float": [I, P, P, L, P],
     "crane_sum_parts": [P, I, L, L, P, L, I, I, P],
-    "crane_gemm_simt": [I, I, P, P, P, P, I, I, I, L, L, L, P],
+    "crane_gemm_simt": [I, I, P, P, P, P, I, I, I, L, L, L, P, P],
+    "crane_gemm_f32_parts": [P, P, P, P, I, I, I, L, L, P, P],
+    "crane_f32_slices": [I, I],
     "crane_gemm_bf16_tcgen05": [P, P, P, P, I, I, I, L, L, L, I, I, I, I, I, L, I, I, I, P, L, P, P],
     "crane_gemm_bf16_pair": [P, P, P, P, I, I, I, L, L, L, I, I, I, I, I, I, L, P, P],
     "crane_paged_attention_simt": [I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, I, P, P, P, P],
@@ -100,10 +102,12 @@ class KernelError(RuntimeError):
 
 class Partials:
     """A matrix product left as ``n`` float partial sums [n, rows, cols] (split
-    along the inner dimension); the consumer adds them up in order."""
+    along the inner dimension); the consumer adds them up in order and rounds
+    once to ``dtype``, the type the product has."""
 
-    def __init__(self, parts: torch.Tensor):
+    def __init__(self, parts: torch.Tensor, dtype: torch.dtype = torch.bfloat16):
         self.parts = parts
+        self.dtype = dtype
 
     @property
     def shape(self):
@@ -356,8 +360,7 @@ class Kernels:
         """x += delta / rms(delta) * w_delta; then, if given, out = x / rms(x) * w_out and
         raw = x in the model dtype.  rms(v) = sqrt(mean(v^2) + eps)."""
         whole, parts, n_parts, stride = _split(delta)
-        dt = out.dtype if out is not None else raw.dtype if raw is not None else (
-            delta.dtype if not isinstance(delta, Partials) else torch.bfloat16)
+        dt = out.dtype if out is not None else raw.dtype if raw is not None else delta.dtype
         self._check(self.lib.crane_add_normed_norm(
             _dt(dt), x.data_ptr(), whole, parts, n_parts, stride, w_delta.data_ptr(), _ptr(w_out), _ptr(out),
             _ptr(raw), x.shape[0], x.shape[1], float(eps_delta), float(eps_out), self._stream(x)), "add_normed_norm")
@@ -738,17 +741,41 @@ class Kernels:
             _dt(out.dtype), aw, ap, an, astr, bw, bp, bn, bstr, wa.data_ptr(), wb.data_ptr(), float(eps),
             out.data_ptr(), out.shape[0], out.shape[1], self._stream(out)), "pair_norm_mean")
 
-    # ---- matrix product on the FP32 cores ------------------------------
-    def gemm_simt(self, a, w, bias, out) -> None:
-        """out[M,N] = a[M,K] @ w[N,K]^T (+ bias); rows may be strided."""
+    # ---- matrix product with 32-bit precision -----------------------------
+    def gemm_simt(self, a, w, bias, out, err=None) -> None:
+        """out[M,N] = a[M,K] @ w[N,K]^T (+ bias); rows may be strided.  Float operands whose rows are whole 16-byte pieces go
+        over the tensor cores, every number as two of 11 bits (``err``: the device-side error word, for waits that run
+        out), everything else over the FP32 cores."""
         M, K = a.shape
         N = w.shape[0]
         assert w.shape[1] == K and out.shape == (M, N)
         assert a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
         self._check(self.lib.crane_gemm_simt(_dt(a.dtype), _dt(out.dtype), a.data_ptr(),
                                              w.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K,
-                                             a.stride(0), w.stride(0), out.stride(0),
+                                             a.stride(0), w.stride(0), out.stride(0), _ptr(err),
                                              self._stream(a)), "gemm_simt")
+
+    @staticmethod
+    @functools.lru_cache(maxsize=8192)
+    def _f32_slices(lib, n: int, k: int) -> int:
+        return lib.crane_f32_slices(n, k)
+
+    def f32_slices(self, n: int, k: int) -> int:
+        """How many slices of the inner dimension a float product has (of its sizes alone, whatever the rows)."""
+        return self._f32_slices(self.lib, n, k)
+
+    def gemm_f32_parts(self, a, w, bias, parts, err) -> bool:
+        """``parts`` [f32_slices, M, N] (float, contiguous): the partial sums of ``gemm_simt``'s result.  False, and nothing
+        done, for operands that the tensor-core kernel does not take: rows that are not whole 16-byte pieces."""
+        M, K = a.shape
+        N = w.shape[0]
+        assert w.shape[1] == K and a.stride(1) == 1 and w.stride(1) == 1 and a.dtype == w.dtype == torch.float32
+        rc = self.lib.crane_gemm_f32_parts(a.data_ptr(), w.data_ptr(), _ptr(bias), parts.data_ptr(), M, N, K, a.stride(0),
+                                           w.stride(0), err.data_ptr(), self._stream(a))
+        if rc == 1:                                       # cudaErrorInvalidValue
+            return False
+        self._check(rc, "gemm_f32_parts")
+        return True
 
     # ---- matrix product on the tensor cores (bfloat16) -------------------
     @staticmethod

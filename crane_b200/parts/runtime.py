@@ -110,12 +110,11 @@ class Runtime:
         result, instead of a buffer called ``name``."""
         M, K = x.shape
         N = w.shape[0]
+        if self.exact:
+            whole = out is not None or (out_dtype is not None and not keep_parts)
+            return self._linear_f32(x, w, bias, name, out, cap, whole, hold)
         if out is None:
             out = self.ws.get(name, M, N, out_dtype or self.dtype, cap)
-        if self.exact:
-            self.kernels.gemm_simt(x, w, bias, out)
-            self.launches += 1
-            return out
         # A product launched straight behind another product (the two branches of a
         # parallel block: output projection, then the feed-forward's first matrix) does not start
         # before that one has finished.  (A prefill of 2,048 tokens that never finished with programmatic dependent
@@ -131,6 +130,36 @@ class Runtime:
             if serial:
                 self.kernels.lib.crane_set_pdl(1)
             self._after_product = self.launches
+
+    def _linear_f32(self, x, w, bias, name: str, out, cap, whole: bool, hold: bool) -> Act:
+        """The product of the 32-bit path.  Few rows: the slices of the inner dimension side by side, left as partial sums
+        unless ``whole``; many fill the SMs without that, and a CTA takes the slices one after the other (the same
+        bits)."""
+        k = self.kernels
+        M, K = x.shape
+        N = w.shape[0]
+        parts = None
+        if M <= self.split_rows:
+            # (16 tiles of weight rows for 148 SMs, as products of hidden 2048 have, take 50 us with a CTA for all slices, 16 side by side)
+            slices = k.f32_slices(N, K)
+            if slices > 1:
+                buf = self.ws.get(f"splitk:{N}:{name}" if hold else f"splitk:{N}", slices * M, N, torch.float32,
+                                  cap=8 * self.split_rows)
+                parts = Partials(buf.view(slices, M, N), torch.float32)
+                if not k.gemm_f32_parts(x, w, bias, parts.parts, self.err):
+                    parts = None
+                elif not whole:
+                    self.launches += 1
+                    return parts
+        if out is None:
+            out = self.ws.get(name, M, N, self.dtype, cap)
+        if parts is not None:
+            k.sum_parts(parts, out)
+            self.launches += 1
+        else:
+            k.gemm_simt(x, w, bias, out, self.err)
+        self.launches += 1
+        return out
 
     def linear_silu_mul(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
         """out[M, N/2] = silu(gate) * up of x @ w^T in one kernel, for w whose rows
@@ -172,8 +201,11 @@ class Runtime:
         for g in range(groups):
             lo, hi = g * group_features, min(N, (g + 1) * group_features)
             x, wg, og = xs[g], w[lo:hi], out[:, lo:hi]
-            if self.exact or not (self.use_tcgen05 and k.tcgen05_takes(x, wg)):
-                k.gemm_simt(x, wg, None, og)
+            if self.exact:
+                self._linear_f32(x, wg, None, name, og, None, True, False)
+                continue
+            if not (self.use_tcgen05 and k.tcgen05_takes(x, wg)):
+                k.gemm_simt(x, wg, None, og, self.err)
                 self.launches += 1
                 continue
             # (behind a product: without programmatic dependent launch, as in ``linear``)

@@ -1102,6 +1102,50 @@ def test_gemm_f32_tiles(K, N, K_):
         assert torch.equal(out[:1], first)               # whatever the batch
 
 
+# partial sums of the 32-bit product, a CTA per slice, add up to the bits of the form that takes the slices in turn: whole and
+# uneven slices, remainders of rows and columns
+@pytest.mark.parametrize("M,N,K_", [(1, 2048, 2048), (17, 130, 1096), (97, 257, 516), (130, 384, 6148)])
+def test_gemm_f32_parts(K, M, N, K_):
+    a, w, bias = torch.randn(M, K_, device=DEV), torch.randn(N, K_, device=DEV), torch.randn(N, device=DEV)
+    whole, err = torch.empty(M, N, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    slices = K.f32_slices(N, K_)
+    assert slices > 1
+    parts = torch.full((slices, M, N), 7.0, device=DEV)
+    assert K.gemm_f32_parts(a, w, bias, parts, err)
+    assert not K.gemm_f32_parts(a[:, 1:5], w[:, 1:5], bias, parts, err)          # (rows that begin between 16-byte pieces)
+    K.gemm_simt(a, w, bias, whole, err)
+    total = parts[0].clone()
+    for s in range(1, slices):
+        total += parts[s]
+    assert torch.equal(total, whole) and int(err.item()) == 0
+    assert rel_err(whole, a.double() @ w.double().T + bias.double()) < acc_tol(K_)
+
+
+# operands that the pieces of the 32-bit product do not carry: infinities, NaN, numbers that round to infinity, beside ordinary
+# rows, with one slice of the inner dimension and with several; numbers near the ends of the range
+@pytest.mark.parametrize("M,N,K_", [(1, 120, 32), (40, 130, 1096), (130, 257, 260)])
+def test_gemm_f32_special_values(K, M, N, K_):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(M)
+    a, w = torch.randn(M, K_, generator=g, device=DEV), torch.randn(N, K_, generator=g, device=DEV)
+    out, bias = torch.empty(M, N, device=DEV), torch.randn(N, generator=g, device=DEV)
+    for scale_a, scale_w in ((1e-30, 1e30), (1e15, 1e-35), (1e18, 1e18)):
+        K.gemm_simt(a * scale_a, w * scale_w, None, out)
+        assert rel_err(out, (a * scale_a).double() @ (w * scale_w).double().T) < acc_tol(K_)
+    a[0, K_ // 2] = math.inf
+    w[3, 1], w[4, 2], w[5, 3], w[6, 4] = -math.inf, math.nan, 3.4028e38, -3.4028e38
+    a[M - 1, 0] = 3.4028e38 if M > 1 else math.inf
+    a[M // 2, 3:5] = 0.25                                 # w[5] and w[6] stay finite there
+    a[0, 3:5] = a[M - 1, 3:5] = 0.0 if M > 1 else 0.25    # (one of those and another of that size or more have no order-free sum)
+    K.gemm_simt(a, w, bias, out)
+    want = a.double() @ w.double().T + bias.double()
+    want32 = want.float()
+    assert torch.equal(torch.isnan(out), torch.isnan(want32)) and torch.equal(torch.isinf(out), torch.isinf(want32))
+    assert torch.equal(out[torch.isinf(out)], want32[torch.isinf(want32)])
+    wrong = (out.double() - want).abs() / (a.double().abs() @ w.double().abs().T).clamp_min(1.0)
+    assert not bool((wrong[torch.isfinite(want32)] > acc_tol(K_)).any())
+
+
 # lengths that differ: one long request among short ones, entries without a row, slices that fill the grid and entries of one
 # slice, groups of one and of several heads, a window, pages smaller than a tile, more entries than lanes
 @pytest.mark.parametrize("nq,nkv,page_size,window,base,most,lens", [
