@@ -170,6 +170,232 @@ paged_attention_simt_kernel(const T* __restrict__ q, T* __restrict__ out,
         if (c < dv) op[c] = from_f32<T>(acc[i] * inv);
     }
 }
+
+// ---- plain softmax attention over float rows, several query rows of a key/value head per CTA ------------------------
+// What bounds it: shared-memory reads (about 1,400 wavefronts a tile of 32 keys), the barriers between a
+// tile's steps and the way of the first tiles from memory.  16
+// query rows (the heads of a group times as many neighbouring tokens as fit) share every key and value that comes in, 32
+// keys at a time by asynchronous copies, one tile ahead; a thread has 2 x 2 scores, then 4 x 4 results.  97 tokens, 16 / 4 heads
+// of 128: 66 us with a warp per (token, head), whose lanes each read a key row of their own, 17 us
+// here (25 when a lane looked up 8 keys one after the other); 2,048 tokens 5,370 / 910, one token behind 8,192 keys 3,070 / 740.
+// Tiles of keys start at multiples of 32 and a row leaves out what is not its own, so that its result does not
+// depend on the rows beside it.  Tokens of several requests in one CTA are taken request by request.
+constexpr int TROWS = 16, TKEYS = 32, TDIM = 128, TPITCH = TDIM + 4;
+
+struct TileParams {
+    const float* q;
+    float* out;
+    const float* k_pool;
+    const float* v_pool;
+    const int* positions;
+    const int* tok_entry;
+    const int* block_table;
+    int max_blocks, num_pages, page_size, n_tokens, nq, nkv, d, dv, v_stride, window;
+    float scale;
+    int sink;
+    const float* sinks;
+    int* err;
+};
+
+__device__ __forceinline__ float half_max(float v) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float half_sum(float v) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+__global__ void __launch_bounds__(128)
+paged_attention_tile_kernel(const TileParams p) {
+    extern __shared__ __align__(16) float tile_smem[];
+    float* q_s = tile_smem;                                      // [TROWS][TPITCH]
+    float* k_s = q_s + TROWS * TPITCH;                           // [2][TKEYS][TPITCH]
+    float* v_s = k_s + 2 * TKEYS * TPITCH;                       // [2][TKEYS][TDIM]
+    float* p_s = v_s + 2 * TKEYS * TDIM;                         // [TROWS][TKEYS]
+    float* corr_s = p_s + TROWS * TKEYS;                         // [TROWS]
+    int* there_s = (int*)(corr_s + TROWS);                       // [2][TKEYS]: the key's page is one of the pool
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int group = p.nq / p.nkv, tokens = TROWS / group, g = blockIdx.x;
+    const int t0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * tokens;              // (later tokens have more keys: they begin)
+    const int d4 = p.d >> 2, dv4 = p.dv >> 2;
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int i = tid; i < TROWS * d4; i += 128) {
+        const int r = i / d4, c = i - r * d4, t = t0 + r / group;
+        const float4 v = r / group < tokens && t < p.n_tokens
+                             ? *(const float4*)(p.q + ((long long)t * p.nq + g * group + r % group) * p.d + 4 * c)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        *(float4*)(q_s + r * TPITCH + 4 * c) = v;
+    }
+    // scores: rows 2 ry and 2 ry + 1, keys kx and kx + 16 of a tile; results: rows 4 warp .. + 3, columns 4 lane .. + 3
+    const int ry = tid >> 4, kx = tid & 15;
+    int pos[2], lo[2], entry[2];
+    float m[2], l[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int r = 2 * ry + i, t = t0 + r / group;
+        const bool mine = r / group < tokens && t < p.n_tokens;
+        entry[i] = mine ? p.tok_entry[t] : -1;
+        pos[i] = mine ? p.positions[t] : -1;
+        lo[i] = p.window > 0 ? max(0, pos[i] - p.window + 1) : 0;
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+    }
+    float4 acc[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    bool bad = false;
+
+    const int t_end = min(t0 + tokens, p.n_tokens);
+    for (int t = t0; t < t_end;) {
+        // a run of tokens of one request: which keys they see
+        const int e = p.tok_entry[t];
+        int from = 0x7fffffff, to = -1, all_from = 0, all_to = 0x7fffffff;       // keys of some token, of every token
+        const bool alone = t == t0;
+        for (; t < t_end && p.tok_entry[t] == e; ++t) {
+            const int at = p.positions[t], begin = p.window > 0 ? max(0, at - p.window + 1) : 0;
+            from = min(from, begin);
+            to = max(to, at);
+            all_from = max(all_from, begin);
+            all_to = min(all_to, at);
+        }
+        const bool one_run = alone && t == t_end;
+        if (e < 0) continue;                                     // rows that pad the step attend to nothing
+        const int* table = p.block_table + (long long)e * p.max_blocks;
+        const int first = from / TKEYS, count = to / TKEYS + 1 - first;
+        auto load = [&](int i) {                                 // tile i of the run
+            float* kt = k_s + (i & 1) * TKEYS * TPITCH;
+            float* vt = v_s + (i & 1) * TKEYS * TDIM;
+            // every lane looks up a key of the tile, so that the look-ups take the time of one
+            const int j = (first + i) * TKEYS + lane, slot = j / p.page_size;
+            const int page = j <= to ? table[slot] : -1;
+            const bool there = page >= 0 && page < p.num_pages;
+            if (!there && j >= from && j <= to) bad = true;
+            const long long row = there ? ((long long)page * p.nkv + g) * p.page_size + (j - slot * p.page_size) : -1;
+            if (warp == 0) there_s[(i & 1) * TKEYS + lane] = there;
+#pragma unroll
+            for (int r = 0; r < TKEYS / 4; ++r) {
+                const long long mine = __shfl_sync(0xffffffffu, row, 4 * r + warp);
+                const uint32_t bytes = mine >= 0 ? 16 : 0;                       // (0: zeros)
+                const long long from_row = mine >= 0 ? mine : 0;
+                if (lane < d4)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::
+                                 "r"((uint32_t)__cvta_generic_to_shared(kt + (4 * r + warp) * TPITCH + 4 * lane)),
+                                 "l"(p.k_pool + from_row * p.d + 4 * lane), "r"(bytes) : "memory");
+                if (lane < dv4)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::
+                                 "r"((uint32_t)__cvta_generic_to_shared(vt + (4 * r + warp) * TDIM + 4 * lane)),
+                                 "l"(p.v_pool + from_row * p.v_stride + 4 * lane), "r"(bytes) : "memory");
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        __syncthreads();                                         // (nobody reads the run before any more; q_s is there)
+        load(0);
+        for (int i = 0; i < count; ++i) {
+            if (i + 1 < count) load(i + 1);
+            if (i + 1 < count) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            const float* kt = k_s + (i & 1) * TKEYS * TPITCH;
+            const float* vt = v_s + (i & 1) * TKEYS * TDIM;
+            float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+            const float* qa = q_s + 2 * ry * TPITCH;
+            const float* ka = kt + kx * TPITCH;
+#pragma unroll 8
+            for (int c = 0; c < p.d; c += 4) {
+                const float4 q0 = *(const float4*)(qa + c), q1 = *(const float4*)(qa + TPITCH + c);
+                const float4 k0 = *(const float4*)(ka + c), k1 = *(const float4*)(ka + 16 * TPITCH + c);
+                s[0][0] = fmaf(q0.w, k0.w, fmaf(q0.z, k0.z, fmaf(q0.y, k0.y, fmaf(q0.x, k0.x, s[0][0]))));
+                s[0][1] = fmaf(q0.w, k1.w, fmaf(q0.z, k1.z, fmaf(q0.y, k1.y, fmaf(q0.x, k1.x, s[0][1]))));
+                s[1][0] = fmaf(q1.w, k0.w, fmaf(q1.z, k0.z, fmaf(q1.y, k0.y, fmaf(q1.x, k0.x, s[1][0]))));
+                s[1][1] = fmaf(q1.w, k1.w, fmaf(q1.z, k1.z, fmaf(q1.y, k1.y, fmaf(q1.x, k1.x, s[1][1]))));
+            }
+            const int j0 = (first + i) * TKEYS + kx;
+#pragma unroll
+            for (int a = 0; a < 2; ++a) {
+                float w[2];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int j = j0 + 16 * b;
+                    const bool sees = entry[a] == e && j >= lo[a] && j <= pos[a] && there_s[(i & 1) * TKEYS + kx + 16 * b];
+                    w[b] = sees ? s[a][b] * p.scale : -INFINITY;
+                }
+                const float m_new = fmaxf(m[a], half_max(fmaxf(w[0], w[1])));
+#pragma unroll
+                for (int b = 0; b < 2; ++b) w[b] = w[b] == -INFINITY ? 0.f : expf(w[b] - m_new);
+                const float corr = m_new == -INFINITY ? 1.f : m[a] == -INFINITY ? 0.f : expf(m[a] - m_new);
+                l[a] = l[a] * corr + half_sum(w[0] + w[1]);
+                m[a] = m_new;
+                p_s[(2 * ry + a) * TKEYS + kx] = w[0];
+                p_s[(2 * ry + a) * TKEYS + kx + 16] = w[1];
+                if (kx == 0) corr_s[2 * ry + a] = corr;
+            }
+            __syncthreads();
+            if (lane < dv4) {
+                const float* pr = p_s + 4 * warp * TKEYS;
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const float corr = corr_s[4 * warp + a];
+                    acc[a].x *= corr; acc[a].y *= corr; acc[a].z *= corr; acc[a].w *= corr;
+                }
+                // (a weight of 0 leaves a key's values out, whatever they are, in tiles that not every row sees all of)
+                auto values = [&](auto some) {
+#pragma unroll 2
+                    for (int j = 0; j < TKEYS; j += 4) {
+                        float4 w[4];
+#pragma unroll
+                        for (int a = 0; a < 4; ++a) w[a] = *(const float4*)(pr + a * TKEYS + j);
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) {
+                            const float4 v = *(const float4*)(vt + (j + b) * TDIM + 4 * lane);
+#pragma unroll
+                            for (int a = 0; a < 4; ++a) {
+                                const float x = b == 0 ? w[a].x : b == 1 ? w[a].y : b == 2 ? w[a].z : w[a].w;
+                                if (decltype(some)::value && x == 0.f) continue;
+                                acc[a].x = fmaf(x, v.x, acc[a].x);
+                                acc[a].y = fmaf(x, v.y, acc[a].y);
+                                acc[a].z = fmaf(x, v.z, acc[a].z);
+                                acc[a].w = fmaf(x, v.w, acc[a].w);
+                            }
+                        }
+                    }
+                };
+                const int j0 = (first + i) * TKEYS;
+                if (one_run && j0 >= all_from && j0 + TKEYS - 1 <= all_to) values(std::false_type{});
+                else values(std::true_type{});
+            }
+            __syncthreads();                                     // before the tile after next and its weights come here
+        }
+    }
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(p.err, CRANE_ERR_PAGE_RANGE);
+    // what a row's sum is divided by, with the candidates that have no value
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        float sum = l[a];
+        if (p.sink) sum += expf(-m[a]);
+        float inv = sum > 0.f ? 1.f / sum : 0.f;
+        if (p.sinks != nullptr) {
+            const float s = p.sinks[g * group + (2 * ry + a) % group], top = fmaxf(m[a], s), mine = expf(m[a] - top);
+            inv = mine / fmaf(sum, mine, expf(s - top));
+        }
+        __syncwarp();
+        if (kx == 0) corr_s[2 * ry + a] = inv;
+    }
+    __syncthreads();
+    if (lane < dv4) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int r = 4 * warp + a, t = t0 + r / group;
+            if (r / group >= tokens || t >= p.n_tokens || p.tok_entry[t] < 0) continue;
+            const float inv = corr_s[r];
+            *(float4*)(p.out + ((long long)t * p.nq + g * group + r % group) * p.dv + 4 * lane) =
+                make_float4(acc[a].x * inv, acc[a].y * inv, acc[a].z * inv, acc[a].w * inv);
+        }
+    }
+}
 }  // namespace
 
 static int launch_simt(int dtype, const void* q, void* out, const void* k_pool, const void* v_pool,
@@ -181,6 +407,23 @@ static int launch_simt(int dtype, const void* q, void* out, const void* k_pool, 
     if (d > MAXD || d <= 0 || dv > MAXDV || dv <= 0 || v_stride < dv || nkv <= 0 || nq % nkv != 0 ||
         sm.maps < 1 || sm.d_row < (sm.maps - 1) * sm.d_map + d || (out_cross != nullptr && sm.maps != 1))
         return (int)cudaErrorInvalidValue;
+    // Plain softmax over heads of at most 128 elements in whole 16-byte pieces, whose groups fit 16 rows: many rows share what they
+    // read.  (By what the attention is, never by the step: a row's result must not depend on the rows beside it.)
+    const bool plain = dtype == 0 && out_cross == nullptr && sm.maps == 1 && sm.softcap == 0.f && sm.chunk == 0 && !sm.sigmoid &&
+                       sm.out_f32 == nullptr && sm.d_row == d;
+    if (plain && d <= TDIM && dv <= TDIM && (d | dv | v_stride) % 4 == 0 && nq / nkv <= TROWS &&
+        ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % 16 == 0) {
+        const int tokens = TROWS / (nq / nkv);
+        const size_t need = (size_t)(TROWS * TPITCH + 2 * TKEYS * (TPITCH + TDIM) + TROWS * (TKEYS + 1) + 2 * TKEYS) * sizeof(float);
+        const cudaError_t rc = cudaFuncSetAttribute(paged_attention_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+        if (rc != cudaSuccess) { cudaGetLastError(); return (int)rc; }
+        const int tiles = (n_tokens + tokens - 1) / tokens;
+        if (tiles <= 65535) {
+            const TileParams tp{(const float*)q, (float*)out, (const float*)k_pool, (const float*)v_pool, positions, tok_entry, block_table,
+                                max_blocks, num_pages, page_size, n_tokens, nq, nkv, d, dv, v_stride, window, scale, sink, sm.sinks, err};
+            return crane_launch(paged_attention_tile_kernel, dim3(nkv, tiles), dim3(128), need, st, tp);
+        }
+    }
     const size_t smem = (size_t)WARPS * d * sizeof(float);
     const long long warps = (long long)n_tokens * nq * (out_cross != nullptr ? nkv : sm.maps);
     const int blocks = (int)((warps + WARPS - 1) / WARPS);

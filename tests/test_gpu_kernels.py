@@ -1121,6 +1121,44 @@ def test_gemm_f32_parts(K, M, N, K_):
     assert rel_err(whole, a.double() @ w.double().T + bias.double()) < acc_tol(K_)
 
 
+# the 32-bit attention of several rows per CTA: requests that begin within a CTA's tokens, padding rows, groups that fill its 16
+# rows or not, windows, heads of whole 16-byte pieces, values that a row must not read, a row's bits whatever is beside it
+@pytest.mark.parametrize("nq,nkv,d,page_size,window,lens,q_lens", [
+    (16, 4, 128, 64, 0, [97, 5, 130], [97, 1, 40]), (3, 1, 24, 8, 0, [40, 33, 1], [7, 33, 1]), (16, 1, 64, 16, 20, [65, 70], [65, 3]),
+    (4, 4, 128, 32, 33, [200], [150]), (10, 2, 100, 16, 0, [31, 32, 33, 64], [1, 1, 1, 1])])
+def test_paged_attention_tiles(K, err, nq, nkv, d, page_size, window, lens, q_lens):
+    torch.manual_seed(nq * d)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    ks, vs = [torch.randn(n, nkv, d) for n in lens], [torch.randn(n, nkv, d) for n in lens]
+    qs = [torch.randn(n, nq, d) for n in q_lens]
+    k_pool, v_pool, table = paged_cache(ks, vs, page_size, torch.float32)
+    q = torch.cat(qs).to(DEV).reshape(-1, nq * d)
+    pos = [n - m + i for n, m in zip(lens, q_lens) for i in range(m)]
+    ent = [e for e, m in enumerate(q_lens) for _ in range(m)]
+
+    def run(rows, v=v_pool):
+        out = torch.full((len(rows) + 2, nq * d), 7.0, device=DEV)
+        qq = torch.cat([q[rows], q[:2]])
+        K.paged_attention_simt(qq, out, k_pool, v, i32([pos[r] for r in rows] + [0, 0]), i32([ent[r] for r in rows] + [-1, -1]),
+                               table, page_size, nq, nkv, d, window, d ** -0.5, err)
+        assert bool((out[-2:] == 7.0).all())                   # padding rows
+        return out[:-2]
+
+    out = run(list(range(len(pos))))
+    want = _dense_attention(qs, ks, vs, lens, q_lens, nq, nkv, d, window)
+    assert rel_err(out, want) < 4e-6 and int(err.item()) == 0
+    for r in (0, len(pos) // 2, len(pos) - 1):
+        assert torch.equal(run([r])[0], out[r])
+    back = list(range(len(pos)))[::-1]
+    assert torch.equal(run(back), out[back])
+    # the last key's values are nobody's but the last row's of the first request
+    last, at = (lens[0] - 1) // page_size, (lens[0] - 1) % page_size
+    v_pool[table[0, last].long(), :, at] = math.inf
+    again = run(list(range(len(pos))))
+    keep = [r for r in range(len(pos)) if r != q_lens[0] - 1]
+    assert torch.equal(again[keep], out[keep]) and not bool(torch.isfinite(again[q_lens[0] - 1]).any())
+
+
 # operands that the pieces of the 32-bit product do not carry: infinities, NaN, numbers that round to infinity, beside ordinary
 # rows, with one slice of the inner dimension and with several; numbers near the ends of the range
 @pytest.mark.parametrize("M,N,K_", [(1, 120, 32), (40, 130, 1096), (130, 257, 260)])
