@@ -155,8 +155,18 @@ __device__ __forceinline__ void prefetch_l2(const GemmParams& p, int lane) {
     }
 }
 
+// silu(gate) * up.  The result is rounded to bf16: the approximate exp and division (each good to a few units in the last
+// place of a float) are far inside that, and a third as long.
+__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.f + __expf(-g)) * u; }
+
 // OUT_F32: float output (else bf16).  TRANSPOSED: element (a, b) goes to out[b * ld + a].
-template <int BN, int STAGES, bool OUT_F32, bool TRANSPOSED>
+// SILU (transposed, bf16, whole inner dimension): the rows of A (weights) come in blocks of 32 = 16 gate rows, then the 16 up
+// rows of the same features, so a feature's two halves lie 16 lanes apart; element (f, b) = silu(gate) * up goes to
+// out[b * ld + f].  For the few rows of decode steps whose gate/up product has tiles enough for the SMs without slices (16,384
+// and 28,672 rows of weights): a launch in the chain of dependent kernels less.  Whole steps, ms, a kernel of its own behind the
+// product / here: hidden 3072 21 requests 2.83 / 2.75, 1 request 2.08 / 2.00, hidden 4096 4 requests 3.36 / 3.30, 16 requests
+// 3.33 / 3.26.
+template <int BN, int STAGES, bool OUT_F32, bool TRANSPOSED, bool SILU = false>
 __global__ void __launch_bounds__(NUM_THREADS)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const GemmParams p) {
@@ -276,6 +286,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     for (int j = 0; j < 16; ++j) r[j] = 0u;
                 }
                 if (a >= p.rows_a) continue;
+                if (SILU) {
+                    // (rows_a is a multiple of 32: the whole warp is here) two tokens at a time: the gate lanes take one,
+                    // the up lanes the other
+                    const bool upper = lane >= 16;
+                    __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (a0 >> 1) + quarter * 16 + (lane & 15);
+#pragma unroll
+                    for (int j = 0; j < 16; j += 2) {
+                        const float mine = __uint_as_float(upper ? r[j + 1] : r[j]);
+                        const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(upper ? r[j] : r[j + 1]), 16);
+                        const int b = b0 + c0 + j + (upper ? 1 : 0);
+                        if (b < p.rows_b)
+                            dst[(long long)b * p.ld_out] = __float2bfloat16_rn(upper ? silu_mul(other, mine) : silu_mul(mine, other));
+                    }
+                    continue;
+                }
                 if (!TRANSPOSED && !split && b0 + c0 + 16 <= p.rows_b) {
                     // 16 consecutive features of one token: whole 16-byte stores when aligned
                     float v[16];
@@ -384,10 +409,7 @@ __device__ __forceinline__ void store_chunk32(const GemmParams& p, const uint32_
         float v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-            const float g = __uint_as_float(r[j]), u = __uint_as_float(r[16 + j]);
-            // the result is rounded to bf16: the approximate exp and division (each good to a
-            // few units in the last place of a float) are far inside that, and a third as long
-            v[j] = __fdividef(g, 1.f + __expf(-g)) * u;
+            v[j] = silu_mul(__uint_as_float(r[j]), __uint_as_float(r[16 + j]));
         }
 #pragma unroll
         for (int j = 0; j < 16; j += 8) {
@@ -910,11 +932,11 @@ bool make_map(CUtensorMap* map, const void* ptr, int rows, int k, long long ld, 
     return true;
 }
 
-template <int BN, int STAGES, bool OUT_F32, bool TRANSPOSED>
+template <int BN, int STAGES, bool OUT_F32, bool TRANSPOSED, bool SILU = false>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, dim3 grid,
            cudaStream_t st) {
     constexpr size_t smem = STAGES * (BM * BK * 2 + BN * BK * 2) + (2 * STAGES + 1) * 8 + 16 + 1024;
-    auto kern = gemm_bf16_kernel<BN, STAGES, OUT_F32, TRANSPOSED>;
+    auto kern = gemm_bf16_kernel<BN, STAGES, OUT_F32, TRANSPOSED, SILU>;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -1004,7 +1026,7 @@ int dispatch_bn(int bn, const CUtensorMap& ma, const CUtensorMap& mb, const Gemm
 
 // D[a, b] = sum_k A[a, k] B[b, k].  bn: columns (rows of B) per tile, 16..256.
 // tile_rows: 128, or 256 (bf16 output, untransposed, no slices, no epilogue, bn 128 / 192 / 256 only).
-// epilogue: 0 none, 1 silu(gate) * up (see the persistent kernel).
+// epilogue: 0 none, 1 silu(gate) * up (see the persistent kernel; transposed: bn 16, 32 or 64).
 // out_f32 / transposed as in the kernel; split_k > 1 writes float partial sums
 // [split_k][...] into `out` (which must then be float) `split_stride` apart.
 // group_features > 0: grouped activations (see the top of the file): row blocks of `group_rows` rows each, and
@@ -1051,9 +1073,19 @@ CRANE_API int crane_gemm_bf16_tcgen05(const void* A, const void* B, const float*
         return (int)cudaErrorInvalidValue;
     }
     if (tile_rows != BM) return (int)cudaErrorInvalidValue;
+    if (epilogue == 1 && transposed) {
+        // the same for few tokens: the weights are A, bn tokens a tile
+        if (split_k != 1 || out_f32 || bias != nullptr || (rows_a & 31)) return (int)cudaErrorInvalidValue;
+        switch (bn) {
+            case 16: return launch<16, 6, false, true, true>(ma, mb, p, grid, st);
+            case 32: return launch<32, 5, false, true, true>(ma, mb, p, grid, st);
+            case 64: return launch<64, 4, false, true, true>(ma, mb, p, grid, st);
+        }
+        return (int)cudaErrorInvalidValue;
+    }
     if (epilogue == 1) {
         // silu(gate) * up: bf16 output of rows_b / 2 columns; the weights' rows in blocks of 16 + 16
-        if (transposed || split_k != 1 || out_f32 || bias != nullptr || (rows_b & 31) || (ld_out & 7) ||
+        if (split_k != 1 || out_f32 || bias != nullptr || (rows_b & 31) || (ld_out & 7) ||
             ((uintptr_t)out & 15))
             return (int)cudaErrorInvalidValue;
         const int tiles = (int)(grid.x * grid.y);

@@ -957,7 +957,7 @@ class Kernels:
         128-row side of the MMA and ``bn`` (16..256) covers the tokens.  With
         ``split_k`` > 1 ``out`` is float [slices, M, N] of partial sums.
         ``silu_mul``: w's rows come as 16 gate rows then the 16 up rows of the same
-        features, and out[M, N/2] = silu(gate) * up.  ``prefetch``: (address,
+        features, and out[M, N/2] = silu(gate) * up (with ``swap``: ``bn`` 16, 32 or 64).  ``prefetch``: (address,
         bytes) of what the step's next product will stream, asked into L2 by the
         narrow-tile kernel while it runs (a hint; ignored by the other kernels).
         ``tile_rows`` 256: tiles of 256 tokens x ``bn`` (128, 192 or 256) features
@@ -968,7 +968,7 @@ class Kernels:
         M, K = x.shape
         N = w.shape[0]
         if silu_mul:
-            assert out.shape == (M, N // 2) and out.stride(1) == 1 and split_k == 1 and not swap
+            assert out.shape == (M, N // 2) and out.stride(1) == 1 and split_k == 1
             ld, stride = out.stride(0), 0
         elif split_k > 1:
             assert out.dtype == torch.float32 and out.dim() == 3 and out.shape[1:] == (M, N)

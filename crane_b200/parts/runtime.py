@@ -166,10 +166,21 @@ class Runtime:
         alternate 16 gate / 16 up.  False if this step's shape has no such kernel
         (few tokens, where the product is computed in slices)."""
         M = x.shape[0]
-        if self.exact or not self.use_tcgen05 or M <= self.silu_rows or not self.kernels.tcgen05_takes(x, w):
+        if self.exact or not self.use_tcgen05 or not self.kernels.tcgen05_takes(x, w):
             return False
         if w.shape[0] % 32 or out.stride(0) % 8 or out.data_ptr() % 16:
             return False
+        if M <= self.silu_rows:
+            # Where the product is in slices of the inner dimension, its partial sums go to a kernel of their own:
+            # whole tiles with this epilogue were slower at hidden 2048 (96 tiles of weights for 148 SMs).
+            bn, slices = self.kernels.few_rows_plan(M, w.shape[0], x.shape[1], self.num_sms)
+            if slices > 1:
+                return False
+            nxt = self._next_weights(w) if w.is_contiguous() else None
+            self.kernels.gemm_tcgen05(x, w, None, out, self.err, bn=bn, swap=True, silu_mul=True,
+                                      prefetch=nxt if M == 1 else None)       # (as in ``_linear_bf16``)
+            self.launches += 1
+            return True
         pair, rows = self.kernels.pair_plan(M, w.shape[0], x.shape[1], self.num_sms, silu_mul=True)
         if pair:
             self.kernels.gemm_pair(x, w, None, out, self.err, bn=pair, silu_mul=True, tile_rows=rows)

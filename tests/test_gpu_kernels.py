@@ -1159,6 +1159,22 @@ def test_paged_attention_tiles(K, err, nq, nkv, d, page_size, window, lens, q_le
     assert torch.equal(again[keep], out[keep]) and not bool(torch.isfinite(again[q_lens[0] - 1]).any())
 
 
+# silu(gate) * up in the epilogue of the product of few rows: every tile of tokens, remainders of tokens and weight rows (a last
+# tile of 32 rows), an output with longer rows
+@pytest.mark.parametrize("M", [1, 2, 15, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("inter,hidden", [(16, 64), (144, 264), (2064, 512)])
+def test_gemm_silu_mul_few_rows(K, err, M, inter, hidden):
+    torch.manual_seed(M + inter)
+    x = torch.randn(M, hidden, device=DEV).bfloat16()
+    gate, up = (torch.randn(inter, hidden, device=DEV).mul_(hidden ** -0.5).bfloat16() for _ in range(2))
+    w = torch.stack([gate.view(-1, 16, hidden), up.view(-1, 16, hidden)], dim=1).reshape(2 * inter, hidden).contiguous()
+    whole = torch.full((M + 1, inter + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    K.gemm_tcgen05(x, w, None, whole[:M, :inter], err, bn=K.few_rows_tile(M), swap=True, silu_mul=True)
+    g, u = x.double() @ gate.double().T, x.double() @ up.double().T
+    assert rel_err(whole[:M, :inter], torch.nn.functional.silu(g) * u) < 4.5e-3          # (half a unit of bf16, and the sums)
+    assert bool((whole[M] == 7.0).all()) and bool((whole[:, inter:] == 7.0).all()) and int(err.item()) == 0
+
+
 # operands that the pieces of the 32-bit product do not carry: infinities, NaN, numbers that round to infinity, beside ordinary
 # rows, with one slice of the inner dimension and with several; numbers near the ends of the range
 @pytest.mark.parametrize("M,N,K_", [(1, 120, 32), (40, 130, 1096), (130, 257, 260)])
