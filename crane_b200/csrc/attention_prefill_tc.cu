@@ -536,14 +536,12 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             if (store) {
                 if (MODS) gate_row(p, row0 + r_begin + r, h, c0, v);
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    uint4 w;
-                    __nv_bfloat162 b0 = __floats2bfloat162_rn(__uint_as_float(v[i]) * inv, __uint_as_float(v[i + 1]) * inv);
-                    __nv_bfloat162 b1 = __floats2bfloat162_rn(__uint_as_float(v[i + 2]) * inv, __uint_as_float(v[i + 3]) * inv);
-                    __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(v[i + 4]) * inv, __uint_as_float(v[i + 5]) * inv);
-                    __nv_bfloat162 b3 = __floats2bfloat162_rn(__uint_as_float(v[i + 6]) * inv, __uint_as_float(v[i + 7]) * inv);
-                    w.x = *(uint32_t*)&b0; w.y = *(uint32_t*)&b1; w.z = *(uint32_t*)&b2; w.w = *(uint32_t*)&b3;
-                    *(uint4*)(orow + c0 + i) = w;
+                for (int i = 0; i < 32; i += 16) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        w[q] = bf16x2_bits(__uint_as_float(v[i + 2 * q]) * inv, __uint_as_float(v[i + 2 * q + 1]) * inv);
+                    store32(orow + c0 + i, w);
                 }
             }
         }
@@ -850,14 +848,12 @@ prefill_attn_tc_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if (store) {
                     if (MODS) gate_row(p, row0 + r_begin + r, h_a + x, c0, o);
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint4 w;
-                        __nv_bfloat162 b0 = __floats2bfloat162_rn(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-                        __nv_bfloat162 b1 = __floats2bfloat162_rn(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-                        __nv_bfloat162 b2 = __floats2bfloat162_rn(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-                        __nv_bfloat162 b3 = __floats2bfloat162_rn(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-                        w.x = *(uint32_t*)&b0; w.y = *(uint32_t*)&b1; w.z = *(uint32_t*)&b2; w.w = *(uint32_t*)&b3;
-                        *(uint4*)(orow + c0 + i) = w;
+                    for (int i = 0; i < 32; i += 16) {
+                        uint32_t w[8];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            w[q] = bf16x2_bits(__uint_as_float(o[i + 2 * q]) * inv, __uint_as_float(o[i + 2 * q + 1]) * inv);
+                        store32(orow + c0 + i, w);
                     }
                 }
             }

