@@ -415,8 +415,12 @@ static int launch_simt(int dtype, const void* q, void* out, const void* k_pool, 
         ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_pool | (uintptr_t)v_pool) % 16 == 0) {
         const int tokens = TROWS / (nq / nkv);
         const size_t need = (size_t)(TROWS * TPITCH + 2 * TKEYS * (TPITCH + TDIM) + TROWS * (TKEYS + 1) + 2 * TKEYS) * sizeof(float);
-        const cudaError_t rc = cudaFuncSetAttribute(paged_attention_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
-        if (rc != cudaSuccess) { cudaGetLastError(); return (int)rc; }
+        static bool configured = false;
+        if (!configured) {
+            const cudaError_t rc = cudaFuncSetAttribute(paged_attention_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+            if (rc != cudaSuccess) { cudaGetLastError(); return (int)rc; }
+            configured = true;
+        }
         const int tiles = (n_tokens + tokens - 1) / tokens;
         if (tiles <= 65535) {
             const TileParams tp{(const float*)q, (float*)out, (const float*)k_pool, (const float*)v_pool, positions, tok_entry, block_table,

@@ -28,8 +28,8 @@
 // beside 128 rows' sums.  One thread for all products, or operands cut by the threads that also fetch them through registers: 1,700
 // to 1,900.  The slices of the inner dimension as clusters that add up through distributed shared memory: 5 to 8 us more per product,
 // and a cluster size that suits many rows, of which one CTA fits an SM, does not suit few.  97 rows, us, before / now: 12288 x 2048
-// 177 / 53, 3072 x 2048 49 / 18, 2048 x 2048 63 / 16, 2048 x 6144 170 / 29 (the weights from DRAM: 15, 4, 3, 8); 16 rows: 40 / 24,
-// 29 / 13, 17 / 11, 43 / 23; one row: 22 / 23, 13 / 12, 12 / 10, 22 / 22.
+// 177 / 53, 3072 x 2048 49 / 18, 2048 x 2048 63 / 16, 2048 x 6144 170 / 29 (the weights from DRAM: 15, 4, 3, 8); 16 rows: 40 / 22,
+// 29 / 12, 17 / 11, 43 / 22; one row: 22 / 21, 13 / 11, 12 / 9, 22 / 21.
 //
 // y = x W^T + b with W stored [out, in]:
 // crane-core/src/models/hunyuan_dense/modeling.rs:273-330.
@@ -167,8 +167,11 @@ template <int NT> struct Shape {
     static constexpr int FIRST_W = 4 + SUM_WARPS, LAST = FIRST_W + 4 * W_GROUPS, THREADS = 32 * (LAST + 4);
     static constexpr int AST = NT <= 80 ? 3 : 2;
     static constexpr int BST = NT <= 96 ? 4 : 3;
-    static constexpr int RAW = NT <= 16 ? 5 : NT <= 64 ? 8 : 6;
-    static constexpr uint32_t B_PIECE = NT * FK * 4, B_BYTES = 2 * B_PIECE;
+    static constexpr int RAW = NT <= 16 ? 4 : NT <= 64 ? 8 : 6;
+    // Few rows: w1 [x1 | x2] is one instruction of twice the rows, into two accumulators side by side (8 instructions of 46 clocks
+    // a stage instead of 12; one row, us: 12288 x 2048 22.7 -> 20.6, 2048 x 6144 21.9 -> 20.6, a head of 120818 x 2048 207 -> 190).
+    static constexpr bool STACK = NT <= 32;
+    static constexpr uint32_t B_PIECE = NT * FK * 4, B_BYTES = (STACK ? 3 : 2) * B_PIECE;
     static constexpr uint32_t COLS_USED = 3 * NT + AST * 2 * PIECE_COLS;
     static constexpr uint32_t TMEM_COLS = COLS_USED <= 256 ? 256 : 512;
     static constexpr size_t BARS = 2 * RAW + 3 * BST + AST;
@@ -187,7 +190,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sm_w = smem;                                        // [RAW][128 rows][128 bytes], 128-byte swizzle
-    uint8_t* sm_b = smem + RAW * RAW_BYTES;                      // [BST][2 pieces][NT rows][128 bytes], 128-byte swizzle
+    uint8_t* sm_b = smem + RAW * RAW_BYTES;                      // [BST][x1, x2 (, x1)][NT rows][128 bytes], 128-byte swizzle
     uint64_t* raw_full = (uint64_t*)(sm_b + BST * S::B_BYTES);   // [RAW] weights have landed
     uint64_t* raw_empty = raw_full + RAW;        // [RAW] they have been read
     uint64_t* a_full = raw_empty + RAW;          // [BST] a stage's rows of A have landed
@@ -214,12 +217,18 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         for (int s = 0; s < BST; ++s) {
             mbar_init(smem_u32(&a_full[s]), 1);
             mbar_init(smem_u32(&b_full[s]), 4);
-            mbar_init(smem_u32(&done[s]), 2);
+            mbar_init(smem_u32(&done[s]), S::STACK ? 1 : 2);
         }
         for (int s = 0; s < AST; ++s) mbar_init(smem_u32(&ready[s]), 4 + S::SUM_WARPS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // the first weights, which are no kernel's result, before tensor memory is asked for: a kernel that still has it all keeps
+        // this one waiting there
+        for (int i = 0; i < min(mine, RAW); ++i) {
+            mbar_expect_tx(smem_u32(&raw_full[i]), RAW_BYTES);
+            tma_load_2d(smem_u32(sm_w + i * RAW_BYTES), &map_w, smem_u32(&raw_full[i]), (first + i) * FK, n0);
+        }
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -231,15 +240,17 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tm_small = tmem + 2 * NT, tm_pieces = tmem + 3 * NT;      // the sums of w1 x1 at 0 and NT
+    // the two sums of w1 x1 and that of the small products; STACK: the latter between the former, so that it lies beside both
+    const uint32_t tm_small = tmem + (S::STACK ? 1 : 2) * NT, tm_pieces = tmem + 3 * NT;
+    auto tm_main = [&](int i) { return tmem + (uint32_t)((i & 1) * (S::STACK ? 2 : 1) * NT); };
     pdl_launch_dependents();
 
     if (warp == 0) {
-        // ---------------- copies of the weights, which are no kernel's result: nothing to wait for ----------------
+        // ---------------- copies of the weights ----------------
         if (lane == 0) {
-            for (int i = 0; i < mine; ++i) {
+            for (int i = RAW; i < mine; ++i) {
                 const int s = i % RAW;
-                if (i >= RAW && !mbar_wait(smem_u32(&raw_empty[s]), ((i / RAW) & 1) ^ 1, abort_flag)) break;
+                if (!mbar_wait(smem_u32(&raw_empty[s]), ((i / RAW) & 1) ^ 1, abort_flag)) break;
                 mbar_expect_tx(smem_u32(&raw_full[s]), RAW_BYTES);
                 tma_load_2d(smem_u32(sm_w + s * RAW_BYTES), &map_w, smem_u32(&raw_full[s]), (first + i) * FK, n0);
             }
@@ -257,7 +268,26 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
     } else if (warp < 3) {
         // ---------------- products: an accumulator is written by one thread alone ----------------
-        if (lane == 0) {
+        if (S::STACK && warp == 1 && lane == 0) {
+            // Stages take turns with [x1 | x2] -> [sum 0 | small] and [x2 | x1] -> [small | sum 1].  The same additions in the same
+            // order as below: the accumulators begin as zeros, which those who take them out write.
+            const uint32_t two = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(2 * NT >> 3) << 17) | ((uint32_t)(FN >> 4) << 24);
+            const uint32_t one = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(FN >> 4) << 24);
+            for (int i = 0; i < mine; ++i) {
+                const int s = i % AST, bs = i % BST;
+                if (!mbar_wait(smem_u32(&ready[s]), (i / AST) & 1, abort_flag)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a1 = tm_pieces + (uint32_t)(s * 2 * PIECE_COLS), a2 = a1 + PIECE_COLS, to = tmem + (uint32_t)((i & 1) * NT);
+                const uint64_t b1 = smem_desc_sw128(smem_u32(sm_b + bs * S::B_BYTES)), b12 = b1 + (i & 1) * (S::B_PIECE >> 4);
+#pragma unroll
+                for (int kk = 0; kk < FK / 8; ++kk) {
+                    umma_ts(to, a1 + 8 * kk, b12 + 2 * kk, two, 1u);
+                    umma_ts(tm_small, a2 + 8 * kk, b1 + 2 * kk, one, 1u);
+                }
+                umma_commit(smem_u32(&done[bs]));
+            }
+        }
+        if (!S::STACK && lane == 0) {
             const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) |
                                    ((uint32_t)(FN >> 4) << 24);
             int slice = slice0, next = 0;                        // the stage that a slice begins with
@@ -270,15 +300,14 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 const uint32_t a1 = tm_pieces + (uint32_t)(s * 2 * PIECE_COLS), a2 = a1 + PIECE_COLS;
                 const uint64_t b1 = smem_desc_sw128(smem_u32(sm_b + bs * S::B_BYTES)), b2 = b1 + (S::B_PIECE >> 4);
                 if (warp == 1) {
-                    const uint32_t tm_main = tmem + (uint32_t)((i & 1) * NT);
 #pragma unroll
                     for (int kk = 0; kk < FK / 8; ++kk)          // 8 elements: 8 columns, 32 bytes
-                        umma_ts(tm_main, a1 + 8 * kk, b1 + 2 * kk, idesc, kk > 0 ? 1u : 0u);
+                        umma_ts(tm_main(i), a1 + 8 * kk, b1 + 2 * kk, idesc, kk > 0 ? 1u : 0u);
                 } else {
 #pragma unroll
                     for (int kk = 0; kk < FK / 8; ++kk) {
-                        umma_ts(tm_small, a2 + 8 * kk, b1 + 2 * kk, idesc, (!fresh || kk > 0) ? 1u : 0u);
-                        umma_ts(tm_small, a1 + 8 * kk, b2 + 2 * kk, idesc, 1u);
+                        umma_ts(tm_small, a1 + 8 * kk, b2 + 2 * kk, idesc, (!fresh || kk > 0) ? 1u : 0u);
+                        umma_ts(tm_small, a2 + 8 * kk, b1 + 2 * kk, idesc, 1u);
                     }
                 }
                 umma_commit(smem_u32(&done[bs]));
@@ -304,6 +333,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 cut(v[j].w, hi.w, lo.w);
                 sts4(base + j * 2048, hi);
                 sts4(base + S::B_PIECE + j * 2048, lo);
+                if (S::STACK) sts4(base + 2 * S::B_PIECE + j * 2048, hi);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -315,7 +345,6 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         for (int i = group; i < mine; i += S::W_GROUPS) {
             const int s = i % AST, ws = i % RAW, bs = i % BST, before = i - AST;
             if (!mbar_wait_warp(smem_u32(&raw_full[ws]), (i / RAW) & 1, abort_flag)) break;
-            if (!mbar_wait_warp(smem_u32(&b_full[bs]), (i / BST) & 1, abort_flag)) break;
             if (before >= 0 && !mbar_wait_warp(smem_u32(&done[before % BST]), (before / BST) & 1, abort_flag)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t from = smem_u32(sm_w + ws * RAW_BYTES) + row * 128;
@@ -337,10 +366,10 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(smem_u32(&ready[s]));
-                mbar_arrive(smem_u32(&raw_empty[ws]));
-            }
+            if (lane == 0) mbar_arrive(smem_u32(&raw_empty[ws]));
+            // (the rows of A last: the first stages' weights are cut before the kernel before has written them)
+            if (!mbar_wait_warp(smem_u32(&b_full[bs]), (i / BST) & 1, abort_flag)) break;
+            if (lane == 0) mbar_arrive(smem_u32(&ready[s]));
         }
     } else if (warp < S::FIRST_W) {
         // ---------------- sums ----------------
@@ -362,6 +391,19 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 for (int j = 0; j < BATCH; j += 2) add2(acc[(c0 + j) / 2], r[j], r[j + 1]);
             }
         };
+        auto clear = [&](uint32_t at) {                          // these columns = 0
+            const float zeros[16] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < COLS; c += 16) tmem_st16(at + from_lanes + (uint32_t)c, zeros);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        };
+        if (S::STACK) {
+            clear(tm_main(0));
+            clear(tm_main(1));
+            clear(tm_small);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+        }
         if (lane == 0) {                                         // both accumulators are free
             mbar_arrive(smem_u32(&ready[0]));
             mbar_arrive(smem_u32(&ready[1]));
@@ -374,8 +416,12 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             const bool ok = mbar_wait_warp(smem_u32(&done[i % BST]), (i / BST) & 1, abort_flag);
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                take(tmem + (uint32_t)((i & 1) * NT));
-                if (i == last) take(tm_small);
+                take(tm_main(i));
+                if (S::STACK) clear(tm_main(i));
+                if (i == last) {
+                    take(tm_small);
+                    if (S::STACK) clear(tm_small);
+                }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 // (the first products of a slice go into both accumulators: they wait for the end of the slice before)
@@ -471,8 +517,12 @@ int launch_split(const SplitParams& p, cudaStream_t st) {
     CUtensorMap map_w, map_a;
     if (!make_map(&map_w, p.w, p.n, p.k, p.ldw, FN) || !make_map(&map_a, p.a, p.m, p.k, p.lda, NT)) return (int)cudaErrorInvalidValue;
     auto kern = gemm_f32_split_kernel<NT>;
-    const cudaError_t rc = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<NT>::SMEM);
-    if (rc != cudaSuccess) { cudaGetLastError(); return (int)rc; }
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t rc = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<NT>::SMEM);
+        if (rc != cudaSuccess) { cudaGetLastError(); return (int)rc; }
+        configured = true;
+    }
     return crane_launch(kern, dim3(p.part_stride > 0 ? p.slices : 1, (p.n + FN - 1) / FN, (p.m + NT - 1) / NT),
                         dim3(Shape<NT>::THREADS), Shape<NT>::SMEM, st, map_w, map_a, p);
 }

@@ -768,10 +768,12 @@ class Kernels:
         """``parts`` [f32_slices, M, N] (float, contiguous): the partial sums of ``gemm_simt``'s result.  False, and nothing
         done, for operands that the tensor-core kernel does not take: rows that are not whole 16-byte pieces."""
         M, K = a.shape
-        N = w.shape[0]
-        assert w.shape[1] == K and a.stride(1) == 1 and w.stride(1) == 1 and a.dtype == w.dtype == torch.float32
-        rc = self.lib.crane_gemm_f32_parts(a.data_ptr(), w.data_ptr(), _ptr(bias), parts.data_ptr(), M, N, K, a.stride(0),
-                                           w.stride(0), err.data_ptr(), self._stream(a))
+        N, inner = w.shape
+        lda, one = a.stride()
+        ldw, one_w = w.stride()
+        assert inner == K and one == one_w == 1 and a.dtype == w.dtype == torch.float32
+        rc = self.lib.crane_gemm_f32_parts(a.data_ptr(), w.data_ptr(), _ptr(bias), parts.data_ptr(), M, N, K, lda, ldw,
+                                           err.data_ptr(), self._stream(a))
         if rc == 1:                                       # cudaErrorInvalidValue
             return False
         self._check(rc, "gemm_f32_parts")

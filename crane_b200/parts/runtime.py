@@ -57,6 +57,7 @@ class Runtime:
         # the next one's together are at most this much: they must fit L2 beside each other.
         self.prefetch_cap = int(os.environ.get("CRANE_L2_PREFETCH_MB", "80")) << 20
         self.use_prefetch = os.environ.get("CRANE_L2_PREFETCH", "1") != "0"
+        self._part_views = {}        # of the 32-bit products' partial sums, by their sizes
         self._after_product = -1     # the launch count as the last product left it
         self._w_order = []           # (address, bytes) of the step's product weights, in order
         self._w_pos = 0
@@ -131,6 +132,22 @@ class Runtime:
                 self.kernels.lib.crane_set_pdl(1)
             self._after_product = self.launches
 
+    def _f32_parts(self, M: int, N: int, K: int, own: Optional[str]) -> Optional[Partials]:
+        """Where a 32-bit product leaves its partial sums, None for one without.  (Views of the workspace, kept by their sizes:
+        making them takes as long as launching the product, and the 32-bit path's small steps are bound by the host.)"""
+        at = (M, N, K, own)
+        kept = self._part_views.get(at)
+        if kept is None or kept[0] != self.ws.generation:
+            slices, parts = self.kernels.f32_slices(N, K), None
+            if slices > 1:
+                buf = self.ws.get(f"splitk:{N}" if own is None else f"splitk:{N}:{own}", slices * M, N, torch.float32,
+                                  cap=8 * self.split_rows)
+                parts = Partials(buf.view(slices, M, N), torch.float32)
+            if len(self._part_views) >= 4096:
+                self._part_views.clear()
+            kept = self._part_views[at] = (self.ws.generation, parts)
+        return kept[1]
+
     def _linear_f32(self, x, w, bias, name: str, out, cap, whole: bool, hold: bool) -> Act:
         """The product of the 32-bit path.  Few rows: the slices of the inner dimension side by side, left as partial sums
         unless ``whole``; many fill the SMs without that, and a CTA takes the slices one after the other (the same
@@ -141,11 +158,8 @@ class Runtime:
         parts = None
         if M <= self.split_rows:
             # (16 tiles of weight rows for 148 SMs, as products of hidden 2048 have, take 50 us with a CTA for all slices, 16 side by side)
-            slices = k.f32_slices(N, K)
-            if slices > 1:
-                buf = self.ws.get(f"splitk:{N}:{name}" if hold else f"splitk:{N}", slices * M, N, torch.float32,
-                                  cap=8 * self.split_rows)
-                parts = Partials(buf.view(slices, M, N), torch.float32)
+            parts = self._f32_parts(M, N, K, name if hold else None)
+            if parts is not None:
                 if not k.gemm_f32_parts(x, w, bias, parts.parts, self.err):
                     parts = None
                 elif not whole:
