@@ -623,8 +623,11 @@ norm_rope_cache_vec_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_stride
 
 // The same for whole bf16 rows of head size 128, eight lanes per (token, head): a
 // lane owns eight neighbours of the first half and their partners in the second
-// half (16-byte loads and stores), four heads per warp.
-__global__ void rope_norm_cache_d128_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_stride,
+// half (16-byte loads and stores), four heads per warp.  PARTS: rows left as partial sums, which a lane reads four at a time
+// (a prompt of 137 tokens, 24 heads, 4 partial sums, whose 9.4 MB it waits for: whole prompt 2.07 ms with a warp per head and
+// 8-byte loads, 1.97 here, 3.3 us a layer).
+template <bool PARTS>
+__global__ void rope_norm_cache_d128_kernel(const GemmOut<__nv_bfloat16> qkv, int qkv_stride,
                                             const int* __restrict__ positions,
                                             const int* __restrict__ tok_entry,
                                             const int* __restrict__ block_table, int max_blocks,
@@ -648,7 +651,7 @@ __global__ void rope_norm_cache_d128_kernel(const __nv_bfloat16* __restrict__ qk
     const bool live = item < (long long)n_tokens * heads;
     const int t = live ? (int)(item / heads) : 0, h = live ? (int)(item % heads) : 0;
     const int pos = positions[t];
-    const __nv_bfloat16* src = qkv + (long long)t * qkv_stride + (long long)h * D;
+    const long long src = (long long)t * qkv_stride + (long long)h * D;
     __nv_bfloat16* dst = nullptr;
     const float* nw = nullptr;
     bool is_v = false;
@@ -694,11 +697,39 @@ __global__ void rope_norm_cache_d128_kernel(const __nv_bfloat16* __restrict__ qk
     }
     pdl_wait();
     float a[8], b[8];
-    {
+    if (PARTS) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] = b[i] = 0.f;
+        const float* at = qkv.parts + src + 8 * sub;
+        for (int p0 = 0; live && p0 < qkv.n_parts; p0 += 4) {
+            float4 x[4][4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const float4* row = (const float4*)(at + (long long)(p0 + p) * qkv.part_stride);
+                const bool there = p0 + p < qkv.n_parts;
+                x[p][0] = there ? row[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[p][1] = there ? row[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[p][2] = there ? row[HALF / 4] : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[p][3] = there ? row[HALF / 4 + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {                    // (in slice order, as every reader of partial sums)
+                a[0] += x[p][0].x; a[1] += x[p][0].y; a[2] += x[p][0].z; a[3] += x[p][0].w;
+                a[4] += x[p][1].x; a[5] += x[p][1].y; a[6] += x[p][1].z; a[7] += x[p][1].w;
+                b[0] += x[p][2].x; b[1] += x[p][2].y; b[2] += x[p][2].z; b[3] += x[p][2].w;
+                b[4] += x[p][3].x; b[5] += x[p][3].y; b[6] += x[p][3].z; b[7] += x[p][3].w;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            a[i] = __bfloat162float(__float2bfloat16_rn(a[i]));
+            b[i] = __bfloat162float(__float2bfloat16_rn(b[i]));
+        }
+    } else {
         uint4 ra = make_uint4(0, 0, 0, 0), rb = ra;
         if (live) {
-            ra = *(const uint4*)(src + 8 * sub);
-            rb = *(const uint4*)(src + HALF + 8 * sub);
+            ra = *(const uint4*)(qkv.whole + src + 8 * sub);
+            rb = *(const uint4*)(qkv.whole + src + HALF + 8 * sub);
         }
         const __nv_bfloat162* pa = (const __nv_bfloat162*)&ra;
         const __nv_bfloat162* pb = (const __nv_bfloat162*)&rb;
@@ -936,13 +967,15 @@ CRANE_API int crane_rope_norm_cache(int dtype, const void* qkv, const float* qkv
     const long long warps = (long long)n_tokens * heads;
     const int threads = 128;
     const int blocks = (int)((warps * 32 + threads - 1) / threads);
-    if (!general && dtype == 1 && d == 128 && qkv != nullptr && qkv_stride % 8 == 0 && n_tokens >= 32 &&
-        ((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)cos_tab |
+    // (8 lanes per head instead of 32: from 32 tokens on they are enough to fill the SMs)
+    if (!general && dtype == 1 && d == 128 && qkv_stride % 8 == 0 && n_tokens >= 32 && (qkv != nullptr || part_stride % 4 == 0) &&
+        ((uintptr_t)qkv | (uintptr_t)qkv_parts | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)cos_tab |
          (uintptr_t)sin_tab | (uintptr_t)q_norm_w | (uintptr_t)k_norm_w) % 16 == 0) {
         const long long lanes = warps * 8;
-        return crane_launch(rope_norm_cache_d128_kernel, dim3((unsigned)((lanes + 255) / 256)), dim3(256), 0, st,
-                            (const __nv_bfloat16*)qkv, qkv_stride, positions, tok_entry, block_table,
-                            max_blocks, cos_tab, sin_tab, table_len, q_norm_w, k_norm_w, eps,
+        const GemmOut<__nv_bfloat16> src{(const __nv_bfloat16*)qkv, qkv_parts, n_parts, part_stride};
+        const auto kern = qkv_parts != nullptr ? rope_norm_cache_d128_kernel<true> : rope_norm_cache_d128_kernel<false>;
+        return crane_launch(kern, dim3((unsigned)((lanes + 255) / 256)), dim3(256), 0, st, src, qkv_stride, positions,
+                            tok_entry, block_table, max_blocks, cos_tab, sin_tab, table_len, q_norm_w, k_norm_w, eps,
                             (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, num_pages,
                             page_size, n_tokens, nq, nkv, has_kv, rotary, err);
     }

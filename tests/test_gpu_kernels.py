@@ -1175,6 +1175,36 @@ def test_gemm_silu_mul_few_rows(K, err, M, inter, hidden):
     assert bool((whole[M] == 7.0).all()) and bool((whole[:, inter:] == 7.0).all()) and int(err.item()) == 0
 
 
+# the rotary kernel of many tokens over partial sums: the bits of the same kernel over the rounded sums, for less and more than the
+# four partial sums a lane reads at a time, padding rows, with norms and without, one token fewer than the kernel takes
+@pytest.mark.parametrize("n_tok,parts,norm", [(31, 3, True), (32, 1, True), (33, 4, False), (137, 5, True), (70, 8, True)])
+def test_rope_norm_cache_parts(K, err, n_tok, parts, norm):
+    from crane_b200.kernels import Partials
+    torch.manual_seed(n_tok)
+    nq, nkv, d, page_size, live = 6, 2, 128, 16, n_tok - 3
+    cols = (nq + 2 * nkv) * d
+    p = torch.randn(parts, n_tok, cols, device=DEV)
+    total = torch.zeros(n_tok, cols, device=DEV)
+    for x in p:
+        total += x
+    pos = torch.arange(n_tok, dtype=torch.int32, device=DEV)
+    ent = torch.tensor([0] * live + [-1] * 3, dtype=torch.int32, device=DEV)
+    pages = -(-n_tok // page_size)
+    table = torch.randperm(pages, device=DEV).int()[None].contiguous()
+    ang = torch.randn(n_tok, d // 2, device=DEV)
+    w = [1 + 0.1 * torch.randn(d, device=DEV) if norm else None for _ in range(2)]
+    got = []
+    for src in (Partials(p), total.bfloat16()):
+        k_pool = torch.zeros(pages, nkv, page_size, d, device=DEV, dtype=torch.bfloat16)
+        v_pool, q_out = torch.zeros_like(k_pool), torch.zeros(n_tok, nq * d, device=DEV, dtype=torch.bfloat16)
+        K.rope_norm_cache(src, cols, torch.bfloat16, pos, ent, table, ang.cos(), ang.sin(), w[0], w[1], 1e-5, q_out, k_pool,
+                          v_pool, page_size, nq, nkv, d, True, True, err)
+        got.append((q_out, k_pool, v_pool))
+    assert int(err.item()) == 0
+    for a, b in zip(*got):
+        assert torch.equal(a, b) and float(a.float().abs().sum()) > 0
+
+
 # operands that the pieces of the 32-bit product do not carry: infinities, NaN, numbers that round to infinity, beside ordinary
 # rows, with one slice of the inner dimension and with several; numbers near the ends of the range
 @pytest.mark.parametrize("M,N,K_", [(1, 120, 32), (40, 130, 1096), (130, 257, 260)])
