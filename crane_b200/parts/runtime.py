@@ -1,8 +1,10 @@
 """What parts run with: the device, the model dtype, the kernels, long-lived
 buffers, the device-side error word and the matrix product.
 
-Matrix products: on the true 32-bit path always the FP32-core kernel of this
-package (no tensor cores, so no reduced-precision mode can slip in).  On the
+Matrix products: on the true 32-bit path the kernel of this package that cuts
+every 32-bit number into two of 11 bits, so that the tensor cores' products are
+exact and their sums are kept in 32 bits (no product of reduced precision
+anywhere; rows that are not whole 16-byte pieces go to the FP32 cores).  On the
 bfloat16 path the tcgen05 kernel of this package where it takes the shape, and
 otherwise the vendor's library product, which is also what the reference uses
 for every product (Candle's matmul, crane-core/src/models/hunyuan_dense/
@@ -141,7 +143,7 @@ class Runtime:
             slices, parts = self.kernels.f32_slices(N, K), None
             if slices > 1:
                 buf = self.ws.get(f"splitk:{N}" if own is None else f"splitk:{N}:{own}", slices * M, N, torch.float32,
-                                  cap=8 * self.split_rows)
+                                  cap=slices * self.split_rows)
                 parts = Partials(buf.view(slices, M, N), torch.float32)
             if len(self._part_views) >= 4096:
                 self._part_views.clear()
