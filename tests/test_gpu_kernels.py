@@ -1176,12 +1176,12 @@ def test_gemm_silu_mul_few_rows(K, err, M, inter, hidden):
 
 
 # the rotary kernel of many tokens over partial sums: the bits of the same kernel over the rounded sums, for less and more than the
-# four partial sums a lane reads at a time, padding rows, with norms and without, one token fewer than the kernel takes
-@pytest.mark.parametrize("n_tok,parts,norm", [(31, 3, True), (32, 1, True), (33, 4, False), (137, 5, True), (70, 8, True)])
+# four partial sums a lane reads at a time, padding rows, with norms and without; one token fewer than it takes: the general kernel, which adds a head's squares in another order
+@pytest.mark.parametrize("n_tok,parts,norm", [(127, 3, True), (128, 1, True), (129, 4, False), (137, 5, True), (150, 8, True)])
 def test_rope_norm_cache_parts(K, err, n_tok, parts, norm):
     from crane_b200.kernels import Partials
     torch.manual_seed(n_tok)
-    nq, nkv, d, page_size, live = 6, 2, 128, 16, n_tok - 3
+    nq, nkv, d, page_size, live = 24, 4, 128, 16, n_tok - 3
     cols = (nq + 2 * nkv) * d
     p = torch.randn(parts, n_tok, cols, device=DEV)
     total = torch.zeros(n_tok, cols, device=DEV)
@@ -1202,7 +1202,8 @@ def test_rope_norm_cache_parts(K, err, n_tok, parts, norm):
         got.append((q_out, k_pool, v_pool))
     assert int(err.item()) == 0
     for a, b in zip(*got):
-        assert torch.equal(a, b) and float(a.float().abs().sum()) > 0
+        assert torch.equal(a, b) if n_tok >= 128 else rel_err(a, b) < 2.0 ** -7       # (a unit of bf16)
+        assert float(a.float().abs().sum()) > 0
 
 
 # operands that the pieces of the 32-bit product do not carry: infinities, NaN, numbers that round to infinity, beside ordinary
